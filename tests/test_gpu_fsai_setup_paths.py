@@ -1,0 +1,62 @@
+"""FSAI setup kernels at the sizes and patterns where their work split can go
+wrong, bit for bit against the oracle."""
+
+import numpy as np
+import pytest
+import scipy.sparse as ss
+
+from gpu_helpers import host_csr, oracle_csr, to_bsr
+
+pytestmark = pytest.mark.gpu
+
+
+def _spd(kind, n, seed=0):
+    """Diagonally dominant symmetric patterns with scaled diagonals."""
+    rng = np.random.default_rng(seed)
+    if kind == "random":  # ragged rows, the mirrored entry rarely at the mirrored place
+        a = ss.random(n, n, density=min(1.0, 9.0 / n), random_state=rng, format="lil")
+    elif kind == "arrow":  # one long row and column among short ones
+        a = ss.lil_matrix((n, n))
+        a[n // 2, :] = rng.normal(size=n)
+    else:  # band
+        k = min(n - 1, 20)
+        a = ss.diags([rng.normal(size=n - d) for d in range(k + 1)], range(k + 1), format="lil")
+    a = ss.csr_matrix(a)
+    a = a + a.T
+    a.setdiag(0)
+    a.eliminate_zeros()
+    a = a + ss.diags(np.asarray(abs(a).sum(axis=1)).ravel() + 1.0)
+    d = ss.diags(np.exp2(rng.integers(-20, 20, size=n)))
+    return ss.csr_matrix(d @ a @ d)
+
+
+def _same(pre, g, gt):
+    for m, o in ((pre.G, g), (pre.GT, gt)):
+        off, col, val = host_csr(m)
+        np.testing.assert_array_equal(off, o.offsets)
+        np.testing.assert_array_equal(col, o.columns)
+        np.testing.assert_array_equal(val, o.values)
+
+
+@pytest.mark.parametrize("kind", ["random", "arrow", "band"])
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 33, 257])
+def test_equilibration_row_blocks(oracle, kind, n):
+    from warp_preconditioners_gb300 import FSAI
+
+    a = _spd(kind, n)
+    pre = FSAI(to_bsr(a), max_row_size=8, kap_tolerance=0.0)
+    g, gt, _ = oracle.fsai(oracle_csr(oracle, a), width=8, tol=0.0)
+    _same(pre, g, gt)
+
+
+def test_missing_transpose_is_refused():
+    from warp_preconditioners_gb300 import FSAI
+
+    for n, r, c in ((9, 8, 0), (40, 3, 30)):
+        a = ss.lil_matrix(_spd("band", n))
+        a[r, c] = 0.01  # outside the band or inside it, one side only
+        a[c, r] = 0.0
+        a = ss.csr_matrix(a)
+        a.eliminate_zeros()
+        with pytest.raises(Exception, match="structurally symmetric"):
+            FSAI(to_bsr(a), max_row_size=4)
