@@ -910,26 +910,32 @@ fsai_round_factor_kernel(RoundState<T> R, int cur, T tolerance, T pivot_floor) {
   }
 }
 
-// Normalise, validate, sort by column and write the ELL rows of a chunk;
-// a warp per row.
-template <typename T>
+// Normalise, validate, sort by column and write the ELL rows of a chunk; G
+// lanes per row (the width rounded up to 8, 16 or 32), NH support positions
+// per lane.  Bound by FP64 issue: the square root and the divisions take
+// about 25 FP64 instructions whatever the number of busy lanes, so a warp
+// takes as many rows as it has room for.  70^3 Q, width 8 (GB300): 380 us a
+// warp per row, 97 us now.
+template <typename T, int G, int NH>
 __global__ void __launch_bounds__(256)
 fsai_round_finish_kernel(RoundState<T> R, const T* __restrict__ scale, int32_t* ell_cols,
                          T* ell_vals, int32_t* row_counts, int32_t* status) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (j >= R.nc) return;
-  const int flags = R.flags[j];
-  if (flags & 2) return;  // rerun by the warp-per-row kernel
-  const int W = R.W, i = R.r0 + j, size = R.size[j];
-  const T norm = sqrt(R.z[(size_t)j * W]);
-  int my_col[2];
-  T my_val[2];
+  constexpr int kNone = 0x7fffffff;
+  const int lane = threadIdx.x & 31, l = lane % G, group = lane / G;
+  const int j = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 / G) + group;
+  const int W = R.W;
+  bool on = j < R.nc;
+  const int flags = on ? R.flags[j] : 0;
+  on = on && !(flags & 2);  // the others are rerun by the warp-per-row kernel
+  const int i = R.r0 + j, size = on ? R.size[j] : 0;
+  const T norm = sqrt(on ? R.z[(size_t)j * W] : T(1));
+  int my_col[NH];
+  T my_val[NH];
   bool valid = true;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int p = lane + 32 * h;
-    my_col[h] = -1;
+  for (int h = 0; h < NH; ++h) {
+    const int p = l + G * h;
+    my_col[h] = kNone;
     my_val[h] = T(0);
     if (p < size) {
       const int c = R.pat[(size_t)j * W + p];
@@ -941,31 +947,38 @@ fsai_round_finish_kernel(RoundState<T> R, const T* __restrict__ scale, int32_t* 
       if (p == 0 && !(val > T(0))) valid = false;
     }
   }
-  const bool all_valid = __all_sync(0xffffffffu, valid);
-  int rank[2] = {0, 0};
-  for (int q = 0; q < size; ++q) {
-    const int cq = __shfl_sync(0xffffffffu, q < 32 ? my_col[0] : my_col[1], q & 31);
-    rank[0] += (cq < my_col[0]);
-    rank[1] += (cq < my_col[1]);
-  }
-  int32_t* oc = ell_cols + (size_t)i * W;
-  T* ov = ell_vals + (size_t)i * W;
+  const unsigned bad = __ballot_sync(0xffffffffu, !valid);
+  int rank[NH] = {};
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int p = lane + 32 * h;
-    if (p < size) {
-      oc[rank[h]] = my_col[h];
-      ov[rank[h]] = my_val[h];
-    } else if (p < W) {
-      oc[p] = -1;
-      ov[p] = T(0);
+  for (int g = 0; g < NH; ++g)
+    for (int q = 0; q < G; ++q) {
+      const int cq = __shfl_sync(0xffffffffu, my_col[g], q, G);
+#pragma unroll
+      for (int h = 0; h < NH; ++h) rank[h] += cq < my_col[h];
     }
+  if (on) {
+    int32_t* oc = ell_cols + (size_t)i * W;
+    T* ov = ell_vals + (size_t)i * W;
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+      const int p = l + G * h;
+      if (p < size) {
+        oc[rank[h]] = my_col[h];
+        ov[rank[h]] = my_val[h];
+      } else if (p < W) {
+        oc[p] = -1;
+        ov[p] = T(0);
+      }
+    }
+    if (l == 0) row_counts[i] = size;
   }
-  if (lane == 0) {
-    row_counts[i] = size;
-    if (flags & 1) atomicAdd(status + 1, 1);
-    if (!all_valid) atomicAdd(status + 2, 1);
-  }
+  // One count a warp.
+  constexpr unsigned kGroup = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+  const bool row_bad = ((bad >> (group * G)) & kGroup) != 0;
+  const int cut = __popc(__ballot_sync(0xffffffffu, on && l == 0 && (flags & 1)));
+  const int lost = __popc(__ballot_sync(0xffffffffu, on && l == 0 && row_bad));
+  if (lane == 0 && cut) atomicAdd(status + 1, cut);
+  if (lane == 0 && lost) atomicAdd(status + 2, lost);
 }
 
 // ---------------------------------------------------------------------------
@@ -988,15 +1001,22 @@ __global__ void scan_block_kernel(const int32_t* in, int32_t* out, int64_t* bloc
   if (threadIdx.x == 1023) block_sums[blockIdx.x] = buf[1023];
 }
 
+// Exclusive scan of the block sums by one warp, 32 at a time.
 __global__ void scan_sums_kernel(int64_t* sums, int nb, int32_t* out_total, int n) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const int lane = threadIdx.x;
   int64_t run = 0;
-  for (int b = 0; b < nb; ++b) {
-    const int64_t t = sums[b];
-    sums[b] = run;
-    run += t;
+  for (int b = 0; b < nb; b += 32) {
+    const int64_t mine = b + lane < nb ? sums[b + lane] : 0;
+    int64_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (b + lane < nb) sums[b + lane] = run + incl - mine;
+    run += __shfl_sync(0xffffffffu, incl, 31);
   }
-  out_total[n] = (int32_t)run;
+  if (lane == 0) out_total[n] = (int32_t)run;
 }
 
 __global__ void scan_add_kernel(int32_t* out, const int64_t* sums, int n) {
@@ -1055,13 +1075,74 @@ __global__ void scatter_transpose_kernel(int nrow, const int32_t* __restrict__ o
   }
 }
 
-// Insertion sort of each row by column (rows of a transpose are short).
+// Sort of one row by column, in place, by G lanes that hold up to E entries
+// each and count the columns below every one; every lane of the warp calls
+// this (`len` 0: no row).  Returns false, untouched, for rows with more than
+// G E entries.
+template <typename T, int G, int E>
+__device__ __forceinline__ bool sort_row(int b, int len, int32_t* cols, T* vals) {
+  const int l = threadIdx.x % G;
+  const bool fits = len <= G * E;
+  if (!fits) len = 0;
+  const int longest = __reduce_max_sync(0xffffffffu, len);
+  int c[E], rank[E];
+  T v[E];
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    const int e = G * k + l;
+    c[k] = 0x7fffffff;
+    rank[k] = 0;
+    if (e < len) {
+      c[k] = cols[b + e];
+      v[k] = vals[b + e];
+    }
+  }
+  // Equal columns keep their order, as an insertion sort has it.
+#pragma unroll
+  for (int g = 0; g < E; ++g) {
+    if (G * g >= longest) break;
+    const int top = min(G, longest - G * g);
+    for (int q = 0; q < top; ++q) {
+      const int cq = __shfl_sync(0xffffffffu, c[g], q, G);
+#pragma unroll
+      for (int k = 0; k < E; ++k)
+        if (G * k < longest)
+          rank[k] += cq < c[k] || (cq == c[k] && (g < k || (g == k && q < l)));
+    }
+  }
+  __syncwarp();  // every entry is read before any is written
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    if (G * k + l < len) {
+      cols[b + rank[k]] = c[k];
+      vals[b + rank[k]] = v[k];
+    }
+  }
+  return fits;
+}
+
+// Sort of each row by column.  Bound by the latency of reading the rows
+// once; an insertion sort by one thread moves the entries through memory
+// one by one, lanes a row apart.  Eight lanes and up to 64 entries a row
+// where rows average 16 entries or fewer, else a warp and up to 256; longer
+// rows keep the insertion sort.  Transpose of the 45^3 Q's width-48 factor
+// (37 entries a row, GB300): 855 us a thread per row, 161 us now; of the 70^3
+// width-8 factor (8 a row): 127, and 98 us (182 with a warp per row).
 template <typename T>
-__global__ void sort_rows_kernel(int nrow, const int32_t* __restrict__ off, int32_t* cols, T* vals) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrow) return;
-  const int b = off[r], e_end = off[r + 1];
-  for (int e = b + 1; e < e_end; ++e) {
+__global__ void __launch_bounds__(256)
+sort_rows_kernel(int nrow, const int32_t* __restrict__ off, int32_t* cols, T* vals) {
+  const bool narrow = off[nrow] <= 16 * (int64_t)nrow;
+  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t r = narrow ? (int64_t)w * 4 + (threadIdx.x & 31) / 8 : w;
+  int b = 0, len = 0;
+  if (r < nrow) {
+    b = off[r];
+    len = off[r + 1] - b;
+  }
+  const bool done = narrow ? sort_row<T, 8, 8>(b, len, cols, vals)
+                           : sort_row<T, 32, 8>(b, len, cols, vals);
+  if (done || threadIdx.x % (narrow ? 8 : 32) != 0) return;
+  for (int e = b + 1; e < b + len; ++e) {
     const int c = cols[e];
     const T v = vals[e];
     int q = e;
@@ -1637,8 +1718,14 @@ static int fsai_setup_t(int n, const int32_t* off, const int32_t* col, const T* 
             R, cur, off, col, ahat.as<T>(), ahatT.as<T>(), ovl.as<int32_t>(), stat + 5);
         fsai_round_factor_kernel<T><<<grid_f, ft, factor_smem, st>>>(R, cur, (T)kap, (T)floor_);
       }
-      fsai_round_finish_kernel<T><<<grid_for(R.nc, 8), 256, 0, st>>>(R, scale, ell_cols, ell_vals,
-                                                                     counts, stat);
+      auto finish = [&](auto* kernel, int rows_per_warp) {
+        kernel<<<grid_for(R.nc, 8 * rows_per_warp), 256, 0, st>>>(R, scale, ell_cols, ell_vals,
+                                                                 counts, stat);
+      };
+      if (W <= 8) finish(fsai_round_finish_kernel<T, 8, 1>, 4);
+      else if (W <= 16) finish(fsai_round_finish_kernel<T, 16, 1>, 2);
+      else if (W <= 32) finish(fsai_round_finish_kernel<T, 32, 1>, 1);
+      else finish(fsai_round_finish_kernel<T, 32, 2>, 1);
       GBPC_CUDA_TRY(cudaGetLastError());
     }
     return GBPC_OK;
@@ -1778,7 +1865,7 @@ static int transpose_t(int nrow, int ncol, const int32_t* off, const int32_t* co
   if (nrow > 0)
     scatter_transpose_kernel<T><<<grid_for(nrow, 256), 256, 0, st>>>(nrow, off, col, val,
                                                                     cursor.as<int32_t>(), t_col, t_val);
-  if (ncol > 0) sort_rows_kernel<T><<<grid_for(ncol, 256), 256, 0, st>>>(ncol, t_off, t_col, t_val);
+  if (ncol > 0) sort_rows_kernel<T><<<grid_for(ncol, 8), 256, 0, st>>>(ncol, t_off, t_col, t_val);
   GBPC_CUDA_TRY(cudaGetLastError());
   GBPC_CUDA_TRY(cudaStreamSynchronize(st));
   return GBPC_OK;
