@@ -129,99 +129,196 @@ __device__ __forceinline__ bool keep_entry(int part, int src_row, int c) {
   return part == 0 || (part == 1 && c < src_row) || (part == 2 && c > src_row);
 }
 
-// Stored entries of each output row after the build filters.
-__global__ void sell_length_kernel(int nrow, const int32_t* __restrict__ off,
-                                   const int32_t* __restrict__ col, const int32_t* rows,
-                                   const int32_t* colmap, int part, int32_t* len) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nrow) return;
+// Stored entries of output row r after the build filters.
+__device__ __forceinline__ int row_length(int r, const int32_t* __restrict__ off,
+                                          const int32_t* __restrict__ col, const int32_t* rows,
+                                          const int32_t* colmap, int part) {
   const int src = rows ? rows[r] : r;
+  if (colmap == nullptr && part == 0) return off[src + 1] - off[src];
   int count = 0;
-  if (colmap == nullptr && part == 0) {
-    count = off[src + 1] - off[src];
-  } else {
-    for (int e = off[src]; e < off[src + 1]; ++e) {
-      const int c = col[e];
-      if (!keep_entry(part, src, c)) continue;
-      if (colmap && colmap[c] < 0) continue;
-      ++count;
-    }
+  for (int e = off[src]; e < off[src + 1]; ++e) {
+    const int c = col[e];
+    if (!keep_entry(part, src, c)) continue;
+    if (colmap && colmap[c] < 0) continue;
+    ++count;
   }
-  len[r] = count;
+  return count;
 }
 
-// Rows ordered by decreasing length inside windows of `window` rows (a stable
-// counting sort per window, one thread per window), so that each 32-row slice
-// holds rows of similar length and padding stays small.
 // Rows are sorted by length inside windows when the plain layout would pad
 // more than this fraction.
 constexpr double kSortPadding = 0.10;
 constexpr int kSortWindow = 256;
 
-// Stable sort of each window's rows by length, longest first: one CTA per
-// window, the thread of row r places it at its rank (rows longer than r, or
-// as long and earlier).
+// Lengths of a window's rows after the build filters, their order by length
+// (longest first, stable: a row's rank is the number of rows longer, or as
+// long and earlier) and the width of each 32-row slice in the plain and in
+// the sorted order; one CTA per window.
 __global__ void __launch_bounds__(kSortWindow)
-window_sort_kernel(int nrow, const int32_t* __restrict__ len, int32_t* perm) {
-  __shared__ int sl[kSortWindow];
+sell_layout_kernel(int nrow, const int32_t* __restrict__ off, const int32_t* __restrict__ col,
+                   const int32_t* rows, const int32_t* colmap, int part, int32_t* perm,
+                   int32_t* plain_width, int32_t* sorted_width) {
+  __shared__ int sl[kSortWindow], sorted[kSortWindow];
   const int lo = blockIdx.x * kSortWindow;
-  const int hi = min(nrow, lo + kSortWindow);
+  const int count = min(nrow - lo, kSortWindow);
   const int k = threadIdx.x;
-  sl[k] = lo + k < hi ? len[lo + k] : -1;
+  const int mine = k < count ? row_length(lo + k, off, col, rows, colmap, part) : -1;
+  sl[k] = mine;
+  sorted[k] = 0;
   __syncthreads();
-  if (lo + k >= hi) return;
-  const int mine = sl[k];
-  int rank = 0;
-  for (int q = 0; q < hi - lo; ++q) {
-    const int o = sl[q];
-    rank += (o > mine) || (o == mine && q < k);
-  }
-  perm[lo + rank] = lo + k;
-}
-
-__global__ void sell_width_kernel(int nrow, int nslices, const int32_t* __restrict__ len,
-                                  const int32_t* perm, int64_t* slice_entries) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= nslices) return;
-  int width = 0;
-  for (int l = 0; l < kSlice; ++l) {
-    const int k = s * kSlice + l;
-    if (k >= nrow) break;
-    width = max(width, len[perm ? perm[k] : k]);
-  }
-  slice_entries[s] = (int64_t)width * kSlice;
-}
-
-__global__ void max_kernel(int n, const int32_t* __restrict__ v, int32_t* out) {
-  int m = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    m = max(m, v[i]);
-  atomicMax(out, m);
-}
-
-// Exclusive scan of int64 counts by a single CTA (setup only).
-__global__ void scan_i64_kernel(const int64_t* in, int64_t* out, int n) {
-  __shared__ int64_t carry;
-  __shared__ int64_t buf[1024];
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < n; base += 1024) {
-    const int i = base + threadIdx.x;
-    const int64_t v = (i < n) ? in[i] : 0;
-    buf[threadIdx.x] = v;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      const int64_t t = (threadIdx.x >= o) ? buf[threadIdx.x - o] : 0;
-      __syncthreads();
-      buf[threadIdx.x] += t;
-      __syncthreads();
+  if (k < count) {
+    int rank = 0;
+    for (int q = 0; q < count; ++q) {
+      const int o = sl[q];
+      rank += (o > mine) || (o == mine && q < k);
     }
-    if (i < n) out[i] = carry + buf[threadIdx.x] - v;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry += buf[1023];
-    __syncthreads();
+    perm[lo + rank] = lo + k;
+    sorted[rank] = mine;
   }
-  if (threadIdx.x == 0) out[n] = carry;
+  __syncthreads();
+  const int plain = __reduce_max_sync(0xffffffffu, max(mine, 0));
+  const int ordered = __reduce_max_sync(0xffffffffu, sorted[k]);
+  if (k % kSlice == 0 && k < count) {
+    plain_width[(lo + k) / kSlice] = plain;
+    sorted_width[(lo + k) / kSlice] = ordered;
+  }
+}
+
+// What sell_schedule_kernel tells the host.
+struct SellLayout {
+  int64_t nent;   // entries including padding of the layout chosen
+  int32_t sorted; // 1: rows sorted inside windows
+  int32_t widest; // width of the widest slice (of both layouts)
+};
+
+// Widths up to this are ordered on the device (one count per warp and width
+// in shared memory); wider slices leave the schedule to the host.
+constexpr int kScheduleWidths = 1024;
+
+// Picks the layout (sorted when that stores kSortPadding fewer entries),
+// and writes its slice offsets and its product schedule: the slices by width
+// descending, stable, each entry {slice, width, first entry} as an int4.
+// Rows still sum their entries in storage order; the schedule only decides
+// which warp takes which slice (and so the order of a fused dot product's
+// per-thread partial sums).  One CTA; each warp walks its own segment of the
+// slices three times (sums, offsets and counts, placement), so a stable
+// counting sort needs no atomics.  It replaces two scans by one CTA with 20
+// barriers per 1,024 slices, two reads of the sizes by the host and a sort
+// there (10,719 slices of a 70^3 factor, GB300: 15 us here; a width-8
+// constructor, two layouts, 11.2 ms before both this and the wider finishing
+// passes, 10.6 ms after).
+__global__ void __launch_bounds__(1024)
+sell_schedule_kernel(int nslices, const int32_t* __restrict__ plain_width,
+                     const int32_t* __restrict__ sorted_width, int64_t* slice_ptr, int4* sched,
+                     SellLayout* info) {
+  extern __shared__ int32_t hist[];  // [32][widest + 1]
+  __shared__ int64_t seg_plain[32], seg_sorted[32];
+  __shared__ int seg_widest[32], scan[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int seg = ((nslices + 1023) / 1024) * 32;  // slices per warp
+  const int begin = min(nslices, warp * seg), end = min(nslices, begin + seg);
+  int64_t sum_p = 0, sum_s = 0;
+  int widest = 0;
+  for (int i = begin + lane; i < end; i += 32) {
+    const int wp = plain_width[i], ws = sorted_width[i];
+    sum_p += wp;
+    sum_s += ws;
+    widest = max(widest, max(wp, ws));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum_p += __shfl_xor_sync(0xffffffffu, sum_p, o);
+    sum_s += __shfl_xor_sync(0xffffffffu, sum_s, o);
+  }
+  widest = __reduce_max_sync(0xffffffffu, widest);
+  if (lane == 0) {
+    seg_plain[warp] = sum_p;
+    seg_sorted[warp] = sum_s;
+    seg_widest[warp] = widest;
+  }
+  __syncthreads();
+  int64_t tot_p = 0, tot_s = 0, before_p = 0, before_s = 0;
+  for (int w = 0; w < 32; ++w) {
+    if (w < warp) {
+      before_p += seg_plain[w];
+      before_s += seg_sorted[w];
+    }
+    tot_p += seg_plain[w];
+    tot_s += seg_sorted[w];
+    widest = max(widest, seg_widest[w]);
+  }
+  tot_p *= kSlice;
+  tot_s *= kSlice;
+  const bool use_sorted = (double)tot_s < (double)tot_p * (1.0 - kSortPadding);
+  const int32_t* width = use_sorted ? sorted_width : plain_width;
+  const bool count = widest < kScheduleWidths;
+  const int nw = widest + 1;
+  if (threadIdx.x == 0) {
+    info->nent = use_sorted ? tot_s : tot_p;
+    info->sorted = use_sorted;
+    info->widest = widest;
+    slice_ptr[nslices] = use_sorted ? tot_s : tot_p;
+  }
+  int32_t* mine = hist + (size_t)warp * nw;
+  if (count)
+    for (int q = lane; q < nw; q += 32) mine[q] = 0;
+  __syncwarp();
+  int64_t at = (use_sorted ? before_s : before_p) * kSlice;
+  for (int base = begin; base < end; base += 32) {
+    const int i = base + lane;
+    const int w = i < end ? width[i] : 0;
+    int64_t incl = (int64_t)w * kSlice;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (i < end) slice_ptr[i] = at + incl - (int64_t)w * kSlice;
+    at += __shfl_sync(0xffffffffu, incl, 31);
+    if (count) {
+      const unsigned same = __match_any_sync(0xffffffffu, i < end ? w : -1);
+      if (i < end && lane == __ffs(same) - 1) mine[w] += __popc(same);
+      __syncwarp();
+    }
+  }
+  if (!count) return;  // the same in every thread
+  __syncthreads();
+  // First place of each (width, warp): widths descending, warps ascending.
+  int total = 0;
+  const int w = nw - 1 - (int)threadIdx.x;
+  if (w >= 0)
+    for (int q = 0; q < 32; ++q) total += hist[(size_t)q * nw + w];
+  int incl = total;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) scan[warp] = incl;
+  __syncthreads();
+  int place = incl - total;
+  for (int q = 0; q < warp; ++q) place += scan[q];
+  if (w >= 0)
+    for (int q = 0; q < 32; ++q) {
+      const int c = hist[(size_t)q * nw + w];
+      hist[(size_t)q * nw + w] = place;
+      place += c;
+    }
+  __syncthreads();
+  for (int base = begin; base < end; base += 32) {
+    const int i = base + lane;
+    const int wi = i < end ? width[i] : 0;
+    const unsigned same = __match_any_sync(0xffffffffu, i < end ? wi : -1);
+    if (i < end) {
+      const uint64_t first = (uint64_t)slice_ptr[i];
+      const int pos = mine[wi] + __popc(same & ((1u << lane) - 1u));
+      sched[pos] = make_int4(i, wi, (int)(uint32_t)(first & 0xffffffffu),
+                             (int)(uint32_t)(first >> 32));
+    }
+    __syncwarp();
+    if (i < end && lane == __ffs(same) - 1) mine[wi] += __popc(same);
+    __syncwarp();
+  }
 }
 
 template <typename VI, typename VO>
@@ -294,14 +391,9 @@ static void launch_fill(const Sell& s, int B, const int32_t* off, const int32_t*
       s.slice_ptr.as<int64_t>(), s.cols.as<int32_t>(), s.vals.as<VO>());
 }
 
-// Product schedule: the slices by width descending (stable), each entry
-// {slice, width, first entry} as an int4, built on the host from slice_ptr.
-// Rows still sum their entries in storage order; the schedule only decides
-// which warp takes which slice (and so the order of a fused dot product's
-// per-thread partial sums).
+// The schedule of sell_schedule_kernel, built on the host from slice_ptr
+// (matrices with slices of kScheduleWidths entries a row or more).
 static int build_schedule(Sell& s, cudaStream_t st) {
-  s.sched.release();
-  if (s.nslices == 0) return GBPC_OK;
   std::vector<int64_t> ptr((size_t)s.nslices + 1);
   GBPC_CUDA_TRY(cudaMemcpyAsync(ptr.data(), s.slice_ptr.p, sizeof(int64_t) * ptr.size(),
                                 cudaMemcpyDeviceToHost, st));
@@ -321,10 +413,6 @@ static int build_schedule(Sell& s, cudaStream_t st) {
     tasks[4 * (size_t)i + 2] = (int32_t)(uint32_t)(ubase & 0xffffffffu);
     tasks[4 * (size_t)i + 3] = (int32_t)(uint32_t)(ubase >> 32);
   }
-  int rc = s.sched.alloc(sizeof(int32_t) * tasks.size());
-  if (rc) return rc;
-  if ((rc = s.err.alloc(sizeof(int32_t)))) return rc;
-  GBPC_CUDA_TRY(cudaMemsetAsync(s.err.p, 0, sizeof(int32_t), st));
   GBPC_CUDA_TRY(cudaMemcpyAsync(s.sched.p, tasks.data(), sizeof(int32_t) * tasks.size(),
                                 cudaMemcpyHostToDevice, st));
   GBPC_CUDA_TRY(cudaStreamSynchronize(st));
@@ -349,57 +437,41 @@ int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const
   s.vdtype = out_dtype;
   s.nslices = (nrow_out + kSlice - 1) / kSlice;
   s.perm.release();
+  s.sched.release();
   int rc = s.slice_ptr.alloc(sizeof(int64_t) * (s.nslices + 1));
   if (rc) return rc;
-  DevBuf counts, len, scratch;
-  if ((rc = counts.alloc(sizeof(int64_t) * (s.nslices + 1)))) return rc;
-  if ((rc = len.alloc(sizeof(int32_t) * (nrow_out + 1)))) return rc;
-  if ((rc = scratch.alloc(sizeof(int32_t) * 2))) return rc;
-  GBPC_CUDA_TRY(cudaMemsetAsync(scratch.p, 0, sizeof(int32_t) * 2, st));
-  if (nrow_out > 0) {
-    sell_length_kernel<<<grid_for(nrow_out, kThreads), kThreads, 0, st>>>(
-        nrow_out, off, col, opt.rows, opt.colmap, opt.part, len.as<int32_t>());
-    sell_width_kernel<<<grid_for(s.nslices, kThreads), kThreads, 0, st>>>(
-        nrow_out, s.nslices, len.as<int32_t>(), nullptr, counts.as<int64_t>());
-  }
-  scan_i64_kernel<<<1, 1024, 0, st>>>(counts.as<int64_t>(), s.slice_ptr.as<int64_t>(), s.nslices);
-  GBPC_CUDA_TRY(cudaGetLastError());
-  if (nrow_out > 0)
-    max_kernel<<<std::min(grid_for(nrow_out, kThreads), 1024), kThreads, 0, st>>>(
-        nrow_out, len.as<int32_t>(), scratch.as<int32_t>());
-  GBPC_CUDA_TRY(cudaGetLastError());
-  int32_t maxlen = 0;
-  GBPC_CUDA_TRY(cudaMemcpyAsync(&s.nent, s.slice_ptr.as<int64_t>() + s.nslices, sizeof(int64_t),
-                                cudaMemcpyDeviceToHost, st));
-  GBPC_CUDA_TRY(cudaMemcpyAsync(&maxlen, scratch.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  GBPC_CUDA_TRY(cudaStreamSynchronize(st));
-  // Try rows sorted by length inside windows; keep that layout when it saves
-  // more than kSortPadding of the stored entries.
-  if (nrow_out > kSlice && maxlen > 0) {
-    DevBuf perm, counts2, ptr2;
-    if ((rc = perm.alloc(sizeof(int32_t) * nrow_out))) return rc;
-    if ((rc = counts2.alloc(sizeof(int64_t) * (s.nslices + 1)))) return rc;
-    if ((rc = ptr2.alloc(sizeof(int64_t) * (s.nslices + 1)))) return rc;
-    const int nwin = (nrow_out + kSortWindow - 1) / kSortWindow;
-    window_sort_kernel<<<nwin, kSortWindow, 0, st>>>(nrow_out, len.as<int32_t>(),
-                                                    perm.as<int32_t>());
-    sell_width_kernel<<<grid_for(s.nslices, kThreads), kThreads, 0, st>>>(
-        nrow_out, s.nslices, len.as<int32_t>(), perm.as<int32_t>(), counts2.as<int64_t>());
-    scan_i64_kernel<<<1, 1024, 0, st>>>(counts2.as<int64_t>(), ptr2.as<int64_t>(), s.nslices);
+  DevBuf perm, widths, info;
+  SellLayout h{};
+  if (s.nslices == 0) {
+    GBPC_CUDA_TRY(cudaMemsetAsync(s.slice_ptr.p, 0, sizeof(int64_t), st));
+  } else {
+    if ((rc = s.sched.alloc(sizeof(int4) * (size_t)s.nslices))) return rc;
+    if ((rc = s.err.alloc(sizeof(int32_t)))) return rc;
+    if ((rc = perm.alloc(sizeof(int32_t) * (size_t)nrow_out))) return rc;
+    if ((rc = widths.alloc(sizeof(int32_t) * 2 * (size_t)s.nslices))) return rc;
+    if ((rc = info.alloc(sizeof(SellLayout)))) return rc;
+    GBPC_CUDA_TRY(cudaMemsetAsync(s.err.p, 0, sizeof(int32_t), st));
+    int32_t* plain = widths.as<int32_t>();
+    sell_layout_kernel<<<(nrow_out + kSortWindow - 1) / kSortWindow, kSortWindow, 0, st>>>(
+        nrow_out, off, col, opt.rows, opt.colmap, opt.part, perm.as<int32_t>(), plain,
+        plain + s.nslices);
+    const size_t smem = sizeof(int32_t) * 32 * kScheduleWidths;
+    GBPC_CUDA_TRY(cudaFuncSetAttribute(sell_schedule_kernel,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    sell_schedule_kernel<<<1, 1024, smem, st>>>(s.nslices, plain, plain + s.nslices,
+                                                s.slice_ptr.as<int64_t>(), s.sched.as<int4>(),
+                                                info.as<SellLayout>());
     GBPC_CUDA_TRY(cudaGetLastError());
-    int64_t nent2 = 0;
-    GBPC_CUDA_TRY(cudaMemcpyAsync(&nent2, ptr2.as<int64_t>() + s.nslices, sizeof(int64_t),
-                                  cudaMemcpyDeviceToHost, st));
+    GBPC_CUDA_TRY(cudaMemcpyAsync(&h, info.p, sizeof(h), cudaMemcpyDeviceToHost, st));
     GBPC_CUDA_TRY(cudaStreamSynchronize(st));
-    if ((double)nent2 < (double)s.nent * (1.0 - kSortPadding)) {
+    if (h.sorted) {
       std::swap(s.perm.p, perm.p);
       std::swap(s.perm.bytes, perm.bytes);
-      std::swap(s.slice_ptr.p, ptr2.p);
-      std::swap(s.slice_ptr.bytes, ptr2.bytes);
-      s.nent = nent2;
+      std::swap(s.perm.tally, perm.tally);
     }
+    if (h.widest >= kScheduleWidths && (rc = build_schedule(s, st))) return rc;
   }
-  if ((rc = build_schedule(s, st))) return rc;
+  s.nent = h.nent;
   if ((rc = s.cols.alloc(sizeof(int32_t) * s.nent))) return rc;
   if ((rc = s.vals.alloc(dtype_size(out_dtype) * s.nent * B * B))) return rc;
   if (s.nslices > 0) {
@@ -421,7 +493,9 @@ int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const
 }
 
 // Rows whose stored length exceeds the width of their slice.
-__global__ void sell_fits_kernel(int nrow, const int32_t* __restrict__ len,
+__global__ void sell_fits_kernel(int nrow, const int32_t* __restrict__ off,
+                                 const int32_t* __restrict__ col, const int32_t* rows,
+                                 const int32_t* colmap, int part,
                                  const int32_t* __restrict__ perm,
                                  const int64_t* __restrict__ slice_ptr, int32_t* bad) {
   const int k_row = blockIdx.x * blockDim.x + threadIdx.x;
@@ -429,7 +503,7 @@ __global__ void sell_fits_kernel(int nrow, const int32_t* __restrict__ len,
   const int sl = k_row / kSlice;
   const int r = perm ? perm[k_row] : k_row;
   const int64_t width = (slice_ptr[sl + 1] - slice_ptr[sl]) / kSlice;
-  if (len[r] > width) atomicAdd(bad, 1);
+  if (row_length(r, off, col, rows, colmap, part) > width) atomicAdd(bad, 1);
 }
 
 // New values for an unchanged pattern: the fill pass again over the existing
@@ -443,15 +517,13 @@ int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val
     return GBPC_ERR_ARG;
   }
   if (s.nrow > 0) {
-    DevBuf len, bad;
+    DevBuf bad;
     int rc;
-    if ((rc = len.alloc(sizeof(int32_t) * (s.nrow + 1)))) return rc;
     if ((rc = bad.alloc(sizeof(int32_t)))) return rc;
     GBPC_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int32_t), st));
-    sell_length_kernel<<<grid_for(s.nrow, kThreads), kThreads, 0, st>>>(
-        s.nrow, off, col, opt.rows, opt.colmap, opt.part, len.as<int32_t>());
     sell_fits_kernel<<<grid_for(s.nrow, kThreads), kThreads, 0, st>>>(
-        s.nrow, len.as<int32_t>(), s.perm.p ? s.perm.as<int32_t>() : nullptr,
+        s.nrow, off, col, opt.rows, opt.colmap, opt.part,
+        s.perm.p ? s.perm.as<int32_t>() : nullptr,
         s.slice_ptr.as<int64_t>(), bad.as<int32_t>());
     GBPC_CUDA_TRY(cudaGetLastError());
     int32_t h = 0;
