@@ -122,14 +122,16 @@ enum EpiKind : int {
   EPI_AXPBY = 0,      // z = alpha * acc + beta * y
   EPI_SQLAP_FWD = 1,  // z = aux0 * acc                      (aux0 = 1/mass)
   EPI_SQLAP_BWD = 2,  // z = alpha * (acc + aux0 * aux1) + beta * y  (aux0 = w*mass[free], aux1 = x)
-  EPI_TRI_LOWER = 3,  // z = aux0 - acc                      (aux0 = rhs)
-  EPI_TRI_UPPER = 4,  // z = inv_block(aux1) * (aux0 - acc)  (aux0 = rhs, aux1 = inverse blocks)
+  EPI_TRI_LOWER = 3,  // z = aux0 - acc                      (aux0 = rhs); out2 = inv_block(aux1) z
+  EPI_TRI_UPPER = 4,  // z = alpha * inv_block(aux1) * (aux0 - acc) + beta * y
+                      //                            (aux0 = rhs, aux1 = inverse blocks)
 };
 
 struct EpiHost {
   int kind = EPI_AXPBY;
   const void* aux0 = nullptr;
   const void* aux1 = nullptr;
+  void* out2 = nullptr;  // second output of EPI_TRI_LOWER
   // Walk the slices in reverse pass order (products without a fused dot;
   // the result is the same either way): the second of two back-to-back
   // products over one matrix then starts on the first one's most recently

@@ -317,36 +317,43 @@ struct DiagOp : Operator {
   bool gathers_x() const override { return false; }
 };
 
+// z = alpha * blockdiag(inv) x + beta * y.
+int block_diag_apply(int vdtype, int B, int nrow, const DevBuf& inv, const void* x, const void* y,
+                     void* z, double alpha, double beta, const int* guard, const DotSpec* dot,
+                     cudaStream_t st) {
+  const Reduction red = make_reduction(dot);
+  const int g = elementwise_grid(nrow);
+  const bool unit = alpha == 1.0 && beta == 0.0;
+#define GBPC_BJ(Bv)                                                                            \
+if (vdtype == GBPC_F64 && unit)                                                              \
+  block_diag_apply_kernel<double, Bv, true><<<g, kThreads, 0, st>>>(                         \
+      nrow, inv.as<double>(), (const double*)x, (const double*)y, (double*)z, alpha, beta,    \
+      guard, red);                                                                           \
+else if (vdtype == GBPC_F64)                                                                 \
+  block_diag_apply_kernel<double, Bv><<<g, kThreads, 0, st>>>(                               \
+      nrow, inv.as<double>(), (const double*)x, (const double*)y, (double*)z, alpha, beta,    \
+      guard, red);                                                                           \
+else                                                                                         \
+  block_diag_apply_kernel<float, Bv><<<g, kThreads, 0, st>>>(                                \
+      nrow, inv.as<float>(), (const float*)x, (const float*)y, (float*)z, (float)alpha,       \
+      (float)beta, guard, red);
+  switch (B) {
+    case 1: GBPC_BJ(1) break;
+    case 2: GBPC_BJ(2) break;
+    case 3: GBPC_BJ(3) break;
+    case 4: GBPC_BJ(4) break;
+  }
+#undef GBPC_BJ
+  GBPC_CUDA_TRY(cudaGetLastError());
+  return GBPC_OK;
+}
+
 struct BlockJacobiOp : Operator {
   int nrow = 0, B = 1;
   DevBuf inv;  // [nrow][B][B], vector dtype
   int apply(const void* x, const void* y, void* z, double alpha, double beta, const int* guard,
             const DotSpec* dot, cudaStream_t st) override {
-    const Reduction red = make_reduction(dot);
-    const int g = elementwise_grid(nrow);
-    const bool unit = alpha == 1.0 && beta == 0.0;
-#define GBPC_BJ(Bv)                                                                            \
-  if (vdtype == GBPC_F64 && unit)                                                              \
-    block_diag_apply_kernel<double, Bv, true><<<g, kThreads, 0, st>>>(                         \
-        nrow, inv.as<double>(), (const double*)x, (const double*)y, (double*)z, alpha, beta,    \
-        guard, red);                                                                           \
-  else if (vdtype == GBPC_F64)                                                                 \
-    block_diag_apply_kernel<double, Bv><<<g, kThreads, 0, st>>>(                               \
-        nrow, inv.as<double>(), (const double*)x, (const double*)y, (double*)z, alpha, beta,    \
-        guard, red);                                                                           \
-  else                                                                                         \
-    block_diag_apply_kernel<float, Bv><<<g, kThreads, 0, st>>>(                                \
-        nrow, inv.as<float>(), (const float*)x, (const float*)y, (float*)z, (float)alpha,       \
-        (float)beta, guard, red);
-    switch (B) {
-      case 1: GBPC_BJ(1) break;
-      case 2: GBPC_BJ(2) break;
-      case 3: GBPC_BJ(3) break;
-      case 4: GBPC_BJ(4) break;
-    }
-#undef GBPC_BJ
-    GBPC_CUDA_TRY(cudaGetLastError());
-    return GBPC_OK;
+    return block_diag_apply(vdtype, B, nrow, inv, x, y, z, alpha, beta, guard, dot, st);
   }
   bool gathers_x() const override { return false; }
 };
@@ -356,30 +363,42 @@ struct Bilu0Op : Operator {
   Sell lower, upper;
   DevBuf inv;         // [nrow][B][B], vector dtype
   DevBuf buf[4];      // a, b, c, d
+  // Both triangular solves start from zero, so their first Jacobi sweeps need
+  // no matrix: the lower one gives x itself, the upper one inv a.  Those and
+  // the scaling of the result are folded into the products next to them:
+  // the last lower product also writes inv a, the last upper one writes
+  // z = alpha inv (a - U c) + beta y with the fused dot.  2 (sweeps - 1)
+  // launches an apply instead of 2 sweeps + 1 and two memsets; bound by the
+  // FP64 issue of the 3 x 3 products (9 multiply-adds a block).  Solve of the
+  // 64^3 K (x) C system, three sweeps (GB300): setup and 103 iterations
+  // 26.1 ms before, 21.2 ms now.
   int apply(const void* x, const void* y, void* z, double alpha, double beta, const int* guard,
             const DotSpec* dot, cudaStream_t st) override {
     // alpha == 0 takes the block-diagonal path of the reference, z = beta * y
     // (block_ilu.py:404-406).
     if (alpha == 0.0) return scale_axpby(vdtype, rows, nullptr, x, y, z, 0.0, beta, guard, dot, st);
-    const size_t bytes = dtype_size(vdtype) * rows;
-    void* a = buf[0].p;
-    void* b = buf[1].p;
-    GBPC_CUDA_TRY(cudaMemsetAsync(a, 0, bytes, st));
+    if (sweeps == 1)
+      return block_diag_apply(vdtype, B, nrow, inv, x, y, z, alpha, beta, guard, dot, st);
     int rc;
-    for (int s = 0; s < sweeps; ++s) {
-      EpiHost e{EPI_TRI_LOWER, x, nullptr};
-      if ((rc = sell_spmv(lower, vdtype, a, nullptr, b, 1.0, 0.0, guard, e, nullptr, st))) return rc;
-      std::swap(a, b);
+    const void* a = x;
+    const void* c = buf[2].p;
+    for (int s = 1; s < sweeps; ++s) {
+      EpiHost e{EPI_TRI_LOWER, x, inv.p};
+      e.out2 = s == sweeps - 1 ? buf[2].p : nullptr;
+      void* out = buf[s & 1].p;
+      if ((rc = sell_spmv(lower, vdtype, a, nullptr, out, 1.0, 0.0, guard, e, nullptr, st))) return rc;
+      a = out;
     }
-    void* c = buf[2].p;
-    void* d = buf[3].p;
-    GBPC_CUDA_TRY(cudaMemsetAsync(c, 0, bytes, st));
-    for (int s = 0; s < sweeps; ++s) {
+    for (int s = 1; s < sweeps; ++s) {
       EpiHost e{EPI_TRI_UPPER, a, inv.p};
-      if ((rc = sell_spmv(upper, vdtype, c, nullptr, d, 1.0, 0.0, guard, e, nullptr, st))) return rc;
-      std::swap(c, d);
+      const bool last = s == sweeps - 1;
+      void* out = last ? z : buf[2 + (s & 1)].p;
+      if ((rc = sell_spmv(upper, vdtype, c, y, out, last ? alpha : 1.0, last ? beta : 0.0, guard, e,
+                          last ? dot : nullptr, st)))
+        return rc;
+      c = out;
     }
-    return scale_axpby(vdtype, rows, nullptr, c, y, z, alpha, beta, guard, dot, st);
+    return GBPC_OK;
   }
   bool gathers_x() const override { return false; }
 };

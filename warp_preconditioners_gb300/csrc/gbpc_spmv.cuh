@@ -23,6 +23,7 @@ template <typename A>
 struct EpiDev {
   const A* aux0;
   const A* aux1;
+  A* out2;  // EPI_TRI_LOWER: also receives inv_block(aux1) z (nullptr: none)
 };
 
 template <typename A>
@@ -69,7 +70,7 @@ __device__ __forceinline__ void spmv_finish(const SellView<V>& m, int row, const
         out[r] = ep.aux0[idx] - acc[r];
       }
     }
-    if (EPI == EPI_TRI_UPPER) {
+    if (EPI == EPI_TRI_UPPER || (EPI == EPI_TRI_LOWER && ep.out2 != nullptr)) {
       A t[B];
 #pragma unroll
       for (int r = 0; r < B; ++r) {
@@ -79,7 +80,15 @@ __device__ __forceinline__ void spmv_finish(const SellView<V>& m, int row, const
         t[r] = s2;
       }
 #pragma unroll
-      for (int r = 0; r < B; ++r) out[r] = t[r];
+      for (int r = 0; r < B; ++r) {
+        const int64_t idx = (int64_t)orow * B + r;
+        if (EPI == EPI_TRI_LOWER) {
+          ep.out2[idx] = t[r];
+        } else {
+          out[r] = alpha_one ? t[r] : alpha * t[r];
+          if (!beta_zero) out[r] = fma_t<A>(beta, y[idx], out[r]);
+        }
+      }
     }
 #pragma unroll
     for (int r = 0; r < B; ++r) {
@@ -849,7 +858,7 @@ static void launch_spmv(const Sell& m, const void* x, const void* y, void* z, do
   SellView<V> view{m.nrow, m.nslices, m.slice_ptr.as<int64_t>(), m.cols.as<int32_t>(),
                    m.vals.as<V>(), m.perm.p ? m.perm.as<int32_t>() : nullptr,
                    m.sched.as<int4>(), ep.reverse ? 1 : 0, m.err.as<int>()};
-  EpiDev<A> e{(const A*)ep.aux0, (const A*)ep.aux1};
+  EpiDev<A> e{(const A*)ep.aux0, (const A*)ep.aux1, (A*)ep.out2};
   const int flags = spmv_flags(alpha, beta);
   if (red.w != nullptr)
     launch_variant<B, V, A, EPI, true>(m.variant, view, x, y, z, alpha, beta, flags, guard, e,
