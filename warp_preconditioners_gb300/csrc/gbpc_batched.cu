@@ -1038,6 +1038,8 @@ extern "C" int gbpc_bop_sqlap(int n, const int32_t* off, const int32_t* col, con
   if (!rc) rc = op->tmp.alloc(dtype_size(vector_dtype) * std::max(n, 1) * max_rhs);
   if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = GBPC_ERR_CUDA;
   if (rc) {
+    inv64.release();  // charged to the operator
+    wm64.release();
     delete op;
     return rc;
   }

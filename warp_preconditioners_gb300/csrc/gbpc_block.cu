@@ -15,6 +15,8 @@
 namespace gbpc {
 
 int scan_exclusive_i32(const int32_t* in, int32_t* out, int n, cudaStream_t st);
+int scan_exclusive_i32(const int32_t* in, int32_t* out, int n, void* sums, cudaStream_t st);
+size_t scan_sums_bytes(int n);
 
 namespace {
 
@@ -558,13 +560,19 @@ template <typename T, int B>
 static int bilu0_setup_t(int nrow, const int32_t* off, const int32_t* col, const T* val,
                          int64_t nnz, int factor_sweeps, T relaxation, T tol, T* factors,
                          T* inverse, int32_t* bad_host, cudaStream_t st) {
-  DevBuf rows, diag, bad, other, order, low, low_before;
+  DevBuf work, rows, diag, bad, other, order, low, low_before, sums;
   int rc;
   constexpr int bb = B * B;
-  if ((rc = rows.alloc(sizeof(int32_t) * std::max<int64_t>(nnz, 1)))) return rc;
-  if ((rc = diag.alloc(sizeof(int32_t) * std::max(nrow, 1)))) return rc;
-  if ((rc = bad.alloc(sizeof(int32_t)))) return rc;
-  if ((rc = other.alloc(sizeof(T) * std::max<int64_t>(nnz, 1) * bb))) return rc;
+  const size_t n = (size_t)std::max(nrow, 1), ne = (size_t)std::max<int64_t>(nnz, 1);
+  if ((rc = alloc_group(work, {{&rows, sizeof(int32_t) * ne},
+                               {&diag, sizeof(int32_t) * n},
+                               {&bad, sizeof(int32_t)},
+                               {&other, sizeof(T) * ne * bb},
+                               {&order, sizeof(int32_t) * ne},
+                               {&low, sizeof(int32_t) * n},
+                               {&low_before, sizeof(int32_t) * (n + 1)},
+                               {&sums, scan_sums_bytes(nrow)}})))
+    return rc;
   GBPC_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int32_t), st));
   GBPC_CUDA_TRY(cudaMemsetAsync(inverse, 0, sizeof(T) * (size_t)std::max(nrow, 1) * bb, st));
   int32_t* pb = bad.as<int32_t>();
@@ -581,12 +589,10 @@ static int bilu0_setup_t(int nrow, const int32_t* off, const int32_t* col, const
   T* cur = factors;
   T* nxt = other.as<T>();
   if (nnz > 0) {  // every row has its diagonal block
-    if ((rc = order.alloc(sizeof(int32_t) * nnz))) return rc;
-    if ((rc = low.alloc(sizeof(int32_t) * nrow))) return rc;
-    if ((rc = low_before.alloc(sizeof(int32_t) * ((size_t)nrow + 1)))) return rc;
     sweep_count_kernel<<<grid_for(nrow, 256), 256, 0, st>>>(nrow, off, diag.as<int32_t>(),
                                                            low.as<int32_t>());
-    if ((rc = scan_exclusive_i32(low.as<int32_t>(), low_before.as<int32_t>(), nrow, st))) return rc;
+    if ((rc = scan_exclusive_i32(low.as<int32_t>(), low_before.as<int32_t>(), nrow, sums.p, st)))
+      return rc;
     const int32_t* ord = order.as<int32_t>();
     sweep_order_kernel<<<grid_for(nrow, 256), 256, 0, st>>>(
         nrow, off, diag.as<int32_t>(), low_before.as<int32_t>(), order.as<int32_t>());

@@ -1026,15 +1026,24 @@ __global__ void scan_add_kernel(int32_t* out, const int64_t* sums, int n) {
 
 }  // namespace
 
-int scan_exclusive_i32(const int32_t* in, int32_t* out, int n, cudaStream_t st) {
+// Stream-ordered; `sums` holds scan_sums_bytes(n).
+size_t scan_sums_bytes(int n) { return sizeof(int64_t) * ((size_t)(n + 1023) / 1024 + 1); }
+
+int scan_exclusive_i32(const int32_t* in, int32_t* out, int n, void* sums, cudaStream_t st) {
   const int nb = (n + 1023) / 1024;
-  DevBuf sums;
-  int rc = sums.alloc(sizeof(int64_t) * (nb + 1));
-  if (rc) return rc;
-  if (n > 0) scan_block_kernel<<<nb, 1024, 0, st>>>(in, out, sums.as<int64_t>(), n);
-  scan_sums_kernel<<<1, 32, 0, st>>>(sums.as<int64_t>(), nb, out, n);
-  if (n > 0) scan_add_kernel<<<nb, 1024, 0, st>>>(out, sums.as<int64_t>(), n);
+  int64_t* s = static_cast<int64_t*>(sums);
+  if (n > 0) scan_block_kernel<<<nb, 1024, 0, st>>>(in, out, s, n);
+  scan_sums_kernel<<<1, 32, 0, st>>>(s, nb, out, n);
+  if (n > 0) scan_add_kernel<<<nb, 1024, 0, st>>>(out, s, n);
   GBPC_CUDA_TRY(cudaGetLastError());
+  return GBPC_OK;
+}
+
+int scan_exclusive_i32(const int32_t* in, int32_t* out, int n, cudaStream_t st) {
+  DevBuf sums;
+  int rc = sums.alloc(scan_sums_bytes(n));
+  if (rc) return rc;
+  if ((rc = scan_exclusive_i32(in, out, n, sums.p, st))) return rc;
   GBPC_CUDA_TRY(cudaStreamSynchronize(st));  // `sums` is released on return
   return GBPC_OK;
 }
@@ -1574,12 +1583,13 @@ static int fsai_setup_t(int n, const int32_t* off, const int32_t* col, const T* 
     GBPC_CUDA_TRY(cudaStreamSynchronize(st));
     nnz = last;
   }
-  DevBuf ahat, ahatT, status, ovl;
+  DevBuf work, ahat, ahatT, status, ovl;
   int rc;
-  if ((rc = ahat.alloc(sizeof(T) * std::max<int64_t>(nnz, 1)))) return rc;
-  if ((rc = ahatT.alloc(sizeof(T) * std::max<int64_t>(nnz, 1)))) return rc;
-  if ((rc = status.alloc(sizeof(int32_t) * 8))) return rc;
-  if ((rc = ovl.alloc(sizeof(int32_t) * std::max(n, 1)))) return rc;
+  if ((rc = alloc_group(work, {{&ahat, sizeof(T) * std::max<int64_t>(nnz, 1)},
+                               {&ahatT, sizeof(T) * std::max<int64_t>(nnz, 1)},
+                               {&status, sizeof(int32_t) * 8},
+                               {&ovl, sizeof(int32_t) * std::max(n, 1)}})))
+    return rc;
   GBPC_CUDA_TRY(cudaMemsetAsync(status.p, 0, sizeof(int32_t) * 8, st));
   int32_t* stat = status.as<int32_t>();
   if (n > 0) {
@@ -1666,17 +1676,22 @@ static int fsai_setup_t(int n, const int32_t* off, const int32_t* col, const T* 
     const size_t budget = std::min<size_t>(free_b / 4, (size_t)8 << 30);
     const int64_t cap = std::max<int64_t>(4096, (int64_t)(budget / per_row));
     const int nc = (int)std::min<int64_t>(n, std::min<int64_t>(cap, chunk_rows_limit()));
+    DevBuf state;
     DevBuf b_size, b_nsel, b_flags, b_pat, b_lo, b_cand, b_z, b_v, b_L, b_a, b_l0, b_l1, b_count;
-    if ((rc = b_size.alloc(sizeof(int32_t) * nc)) || (rc = b_nsel.alloc(sizeof(int32_t) * nc)) ||
-        (rc = b_flags.alloc(sizeof(int32_t) * nc)) ||
-        (rc = b_pat.alloc(sizeof(int32_t) * (size_t)nc * W)) ||
-        (rc = b_lo.alloc(sizeof(int32_t) * (size_t)nc * W)) ||
-        (rc = b_cand.alloc(sizeof(int32_t) * (size_t)nc * SE)) ||
-        (rc = b_z.alloc(sizeof(T) * (size_t)nc * W)) || (rc = b_v.alloc(sizeof(T) * (size_t)nc * W)) ||
-        (rc = b_L.alloc(sizeof(T) * (size_t)nc * W * (W + 1) / 2)) ||
-        (rc = b_a.alloc(sizeof(T) * (size_t)nc * W * SE)) ||
-        (rc = b_l0.alloc(sizeof(int32_t) * nc)) || (rc = b_l1.alloc(sizeof(int32_t) * nc)) ||
-        (rc = b_count.alloc(sizeof(int32_t) * 2)))
+    const size_t rows = (size_t)nc;
+    if ((rc = alloc_group(state, {{&b_size, sizeof(int32_t) * rows},
+                                  {&b_nsel, sizeof(int32_t) * rows},
+                                  {&b_flags, sizeof(int32_t) * rows},
+                                  {&b_pat, sizeof(int32_t) * rows * W},
+                                  {&b_lo, sizeof(int32_t) * rows * W},
+                                  {&b_cand, sizeof(int32_t) * rows * SE},
+                                  {&b_z, sizeof(T) * rows * W},
+                                  {&b_v, sizeof(T) * rows * W},
+                                  {&b_L, sizeof(T) * rows * W * (W + 1) / 2},
+                                  {&b_a, sizeof(T) * rows * W * SE},
+                                  {&b_l0, sizeof(int32_t) * rows},
+                                  {&b_l1, sizeof(int32_t) * rows},
+                                  {&b_count, sizeof(int32_t) * 2}})))
       return rc;
     RoundState<T> R;
     R.W = W;
@@ -1853,14 +1868,16 @@ extern "C" int gbpc_fsai_pack(int n, int width, const int32_t* ell_cols, const v
 template <typename T>
 static int transpose_t(int nrow, int ncol, const int32_t* off, const int32_t* col, const T* val,
                        int32_t* t_off, int32_t* t_col, T* t_val, cudaStream_t st) {
-  DevBuf counts, cursor;
+  DevBuf work, counts, cursor, sums;
   int rc;
-  if ((rc = counts.alloc(sizeof(int32_t) * (ncol + 1)))) return rc;
-  if ((rc = cursor.alloc(sizeof(int32_t) * (ncol + 1)))) return rc;
+  if ((rc = alloc_group(work, {{&counts, sizeof(int32_t) * ((size_t)ncol + 1)},
+                               {&cursor, sizeof(int32_t) * ((size_t)ncol + 1)},
+                               {&sums, scan_sums_bytes(ncol)}})))
+    return rc;
   GBPC_CUDA_TRY(cudaMemsetAsync(counts.p, 0, sizeof(int32_t) * (ncol + 1), st));
   if (nrow > 0) count_columns_kernel<<<grid_for(nrow, 256), 256, 0, st>>>(nrow, off, col, counts.as<int32_t>());
   GBPC_CUDA_TRY(cudaGetLastError());
-  if ((rc = scan_exclusive_i32(counts.as<int32_t>(), t_off, ncol, st))) return rc;
+  if ((rc = scan_exclusive_i32(counts.as<int32_t>(), t_off, ncol, sums.p, st))) return rc;
   GBPC_CUDA_TRY(cudaMemcpyAsync(cursor.p, t_off, sizeof(int32_t) * (ncol + 1), cudaMemcpyDeviceToDevice, st));
   if (nrow > 0)
     scatter_transpose_kernel<T><<<grid_for(nrow, 256), 256, 0, st>>>(nrow, off, col, val,
@@ -1984,10 +2001,11 @@ template <typename T, typename S>
 static int refit_t(int n, const int32_t* a_off, const int32_t* a_col, const T* a_val,
                    const int32_t* g_off, const int32_t* g_col, int width, double floor_, S* out,
                    int32_t* status_host, cudaStream_t st) {
-  DevBuf scale, status;
+  DevBuf work, scale, status;
   int rc;
-  if ((rc = scale.alloc(sizeof(T) * std::max(n, 1)))) return rc;
-  if ((rc = status.alloc(sizeof(int32_t) * 2))) return rc;
+  if ((rc = alloc_group(work, {{&scale, sizeof(T) * std::max(n, 1)},
+                               {&status, sizeof(int32_t) * 2}})))
+    return rc;
   GBPC_CUDA_TRY(cudaMemsetAsync(status.p, 0, sizeof(int32_t) * 2, st));
   int32_t* stat = status.as<int32_t>();
   if (n > 0) {
@@ -2011,9 +2029,10 @@ static int refit_t(int n, const int32_t* a_off, const int32_t* a_col, const T* a
       const int nc = (int)std::min<int64_t>(
           n, std::min<int64_t>(std::max<int64_t>(4096, (int64_t)(budget / (sizeof(T) * tri))),
                                chunk_rows_limit()));
-      DevBuf bins, order, lbuf;
-      if ((rc = bins.alloc(sizeof(int32_t) * (width + 1))) ||
-          (rc = order.alloc(sizeof(int32_t) * n)) || (rc = lbuf.alloc(sizeof(T) * tri * nc)))
+      DevBuf wide, bins, order, lbuf;
+      if ((rc = alloc_group(wide, {{&bins, sizeof(int32_t) * (width + 1)},
+                                   {&order, sizeof(int32_t) * (size_t)n},
+                                   {&lbuf, sizeof(T) * tri * nc}})))
         return rc;
       GBPC_CUDA_TRY(cudaMemsetAsync(bins.p, 0, sizeof(int32_t) * (width + 1), st));
       support_size_count_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, g_off, width,

@@ -554,6 +554,7 @@ struct Gmres {
   Operator* M = nullptr;
   int64_t n = 0;
   int m = 31;
+  DevBuf store;  // of the buffers below
   DevBuf V, w, t, d, vcur, state, work, partials, counter;
   ReduceBuf rb;
   cudaGraphExec_t exec = nullptr;
@@ -840,15 +841,15 @@ extern "C" int gbpc_gmres_create(gbpc_op* A, gbpc_op* M, int restart, void* stre
   g.n = a->rows;
   g.m = restart;
   const size_t vec = sizeof(double) * std::max<int64_t>(g.n, 1);
-  int rc = g.V.alloc(vec * (restart + 1));
-  if (!rc) rc = g.w.alloc(vec);
-  if (!rc) rc = g.t.alloc(vec);
-  if (!rc) rc = g.d.alloc(vec);
-  if (!rc) rc = g.vcur.alloc(vec);
-  if (!rc) rc = g.state.alloc(sizeof(GmresState));
-  if (!rc) rc = g.work.alloc(sizeof(double) * Gmres::work_doubles(restart));
-  if (!rc) rc = g.partials.alloc(sizeof(double) * (size_t)kGCtas * kGMaxK);
-  if (!rc) rc = g.counter.alloc(sizeof(unsigned int));
+  int rc = alloc_group(g.store, {{&g.V, vec * (restart + 1)},
+                                 {&g.w, vec},
+                                 {&g.t, vec},
+                                 {&g.d, vec},
+                                 {&g.vcur, vec},
+                                 {&g.state, sizeof(GmresState)},
+                                 {&g.work, sizeof(double) * Gmres::work_doubles(restart)},
+                                 {&g.partials, sizeof(double) * (size_t)kGCtas * kGMaxK},
+                                 {&g.counter, sizeof(unsigned int)}});
   if (!rc) rc = g.rb.init((cudaStream_t)stream);
   cudaStream_t st = (cudaStream_t)stream;
   if (!rc && (cudaMemsetAsync(g.counter.p, 0, sizeof(unsigned int), st) != cudaSuccess ||

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <memory>
 #include <vector>
 
@@ -53,27 +54,40 @@ struct PdlScope {
   PdlScope& operator=(const PdlScope&) = delete;
 };
 
-// Owned device allocation.
+// Owned device allocation, or (alloc_group) a part of another one.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   size_t* tally = nullptr;  // counter charged with `bytes` (nullable)
+  bool part = false;        // memory of another DevBuf
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
   void release() {
-    if (p) {
+    if (p && !part) {
       cudaFree(p);
       note_release(bytes, tally);
     }
     p = nullptr;
     bytes = 0;
     tally = nullptr;
+    part = false;
   }
   int alloc(size_t n);
   template <typename T> T* as() const { return static_cast<T*>(p); }
 };
+
+// One allocation, owned by `store`, for several buffers, which become parts
+// of it (256-byte aligned) and must not outlive it.  A cudaMalloc and
+// cudaFree pair costs the host 70-130 us on this platform whatever its size
+// (GB300 with Grace; up to 100 MB), and a width-8 FSAI constructor made 45 of
+// them, most of its time outside its kernels.
+struct DevPart {
+  DevBuf* buf;
+  size_t bytes;
+};
+int alloc_group(DevBuf& store, std::initializer_list<DevPart> parts);
 
 // Sliced ELL matrix (32 block rows per slice) with owned storage.
 struct Sell {
@@ -86,9 +100,11 @@ struct Sell {
   DevBuf slice_ptr;  // int64[nslices + 1]
   DevBuf cols;       // int32[nent]
   DevBuf vals;       // vdtype[nent * B * B]
+  DevBuf store;      // the allocation that the buffers here are parts of
   DevBuf perm;       // int32[nrow] when rows are stored sorted by length
   DevBuf sched;      // int4[nslices]: product schedule, slices by width descending
   DevBuf err;        // int32[1]: set by a product kernel whose bounded wait gave up
+  DevBuf misfit;     // int32[1]: rows that do not fit, counted by sell_refill
   int variant = 0;   // product kernel variant chosen by sell_autotune
   int64_t nnz = 0;   // stored entries without padding
 };
@@ -143,6 +159,7 @@ struct ReductionHost;  // defined in gbpc_common.cuh as gbpc::Reduction
 
 // Scratch for one deterministic reduction: partials + arrival counter.
 struct ReduceBuf {
+  DevBuf store;
   DevBuf partials;  // double[kMaxCtas]
   DevBuf counter;   // unsigned int[1], zero between uses
   int init(cudaStream_t st);

@@ -546,6 +546,7 @@ struct Solver {
   bool coop = false;
   int coop_cluster = 0;  // CTAs of that cluster
   coop::Args cargs{};
+  DevBuf store;  // of r .. ks
   DevBuf r, z, p, Ap, Az, y, ks, zeros, t, u;
   ReduceBuf rb;
   // Cached graph for the last (b, x) pair.
@@ -922,13 +923,14 @@ extern "C" int gbpc_solver_create(int method, gbpc_op* A, gbpc_op* M, int use_gr
   s.use_graph = use_graph != 0;
   if (unroll > 0) s.unroll = unroll > 64 ? 64 : unroll;
   const size_t bytes = sizeof(double) * std::max<int64_t>(s.n, 1);
-  int rc = s.r.alloc(bytes);
-  if (!rc) rc = s.z.alloc(bytes);
-  if (!rc) rc = s.p.alloc(bytes);
-  if (!rc) rc = s.Ap.alloc(bytes);
-  if (!rc && method == GBPC_CR) rc = s.Az.alloc(bytes);
-  if (!rc && method == GBPC_CR) rc = s.y.alloc(bytes);
-  if (!rc) rc = s.ks.alloc(sizeof(KrylovScalars));
+  const size_t cr = method == GBPC_CR ? bytes : 0;
+  int rc = alloc_group(s.store, {{&s.r, bytes},
+                                 {&s.z, bytes},
+                                 {&s.p, bytes},
+                                 {&s.Ap, bytes},
+                                 {&s.Az, cr},
+                                 {&s.y, cr},
+                                 {&s.ks, sizeof(KrylovScalars)}});
   if (!rc) rc = s.rb.init((cudaStream_t)stream);
   if (!rc && cudaMemsetAsync(s.ks.p, 0, sizeof(KrylovScalars), (cudaStream_t)stream) != cudaSuccess)
     rc = GBPC_ERR_CUDA;

@@ -266,6 +266,7 @@ struct SqlapOp : Operator {
   Sell fwd;       // L with columns mapped to compact free indices (not built when identity_free)
   Sell bwd;       // rows L[free, :]
   Sell bnd;       // L with only constrained columns (rhs)
+  DevBuf store;  // of the buffers below
   DevBuf inv_mass, wmass, tmp, index, free_idx, zeros;
   int apply(const void* x, const void* y, void* z, double alpha, double beta, const int* guard,
             const DotSpec* dot, cudaStream_t st) override {
@@ -361,6 +362,7 @@ struct BlockJacobiOp : Operator {
 struct Bilu0Op : Operator {
   int nrow = 0, B = 1, sweeps = 1;
   Sell lower, upper;
+  DevBuf store;       // of the buffers below
   DevBuf inv;         // [nrow][B][B], vector dtype
   DevBuf buf[4];      // a, b, c, d
   // Both triangular solves start from zero, so their first Jacobi sweeps need
@@ -608,19 +610,22 @@ extern "C" int gbpc_op_sqlap(int n, const int32_t* offsets, const int32_t* colum
   op->nfree = nfree;
   const size_t vs = dtype_size(dtype);
   int rc = GBPC_OK;
-  DevBuf status, bmap;
+  DevBuf work, status, bmap;
   auto fail = [&](int code) {
+    work.release();  // charged to the operator
     delete op;
     return code;
   };
-  if ((rc = status.alloc(sizeof(int32_t) * 4))) return fail(rc);
-  if ((rc = op->index.alloc(sizeof(int32_t) * std::max(n, 1)))) return fail(rc);
-  if ((rc = op->free_idx.alloc(sizeof(int32_t) * std::max(nfree, 1)))) return fail(rc);
-  if ((rc = op->inv_mass.alloc(vs * std::max(n, 1)))) return fail(rc);
-  if ((rc = op->wmass.alloc(vs * std::max(nfree, 1)))) return fail(rc);
-  if ((rc = op->zeros.alloc(vs * std::max(nfree, 1)))) return fail(rc);
-  if ((rc = op->tmp.alloc(vs * std::max(n, 1)))) return fail(rc);
-  if ((rc = bmap.alloc(sizeof(int32_t) * std::max(n, 1)))) return fail(rc);
+  if ((rc = alloc_group(work, {{&status, sizeof(int32_t) * 4},
+                               {&bmap, sizeof(int32_t) * std::max(n, 1)}})))
+    return fail(rc);
+  if ((rc = alloc_group(op->store, {{&op->index, sizeof(int32_t) * std::max(n, 1)},
+                                    {&op->free_idx, sizeof(int32_t) * std::max(nfree, 1)},
+                                    {&op->inv_mass, vs * std::max(n, 1)},
+                                    {&op->wmass, vs * std::max(nfree, 1)},
+                                    {&op->zeros, vs * std::max(nfree, 1)},
+                                    {&op->tmp, vs * std::max(n, 1)}})))
+    return fail(rc);
   if (cudaMemsetAsync(status.p, 0, sizeof(int32_t) * 4, st) != cudaSuccess ||
       cudaMemsetAsync(op->index.p, 0xff, sizeof(int32_t) * std::max(n, 1), st) != cudaSuccess ||
       cudaMemsetAsync(op->zeros.p, 0, vs * std::max(nfree, 1), st) != cudaSuccess) {
@@ -719,6 +724,7 @@ extern "C" int gbpc_op_diagonal(int nrow, int block, const int32_t* offsets,
   int rc = tmp.alloc(sizeof(double) * std::max<int64_t>(op->rows, 1));
   if (!rc) rc = op->inv.alloc(dtype_size(dtype) * std::max<int64_t>(op->rows, 1));
   if (rc) {
+    tmp.release();  // charged to the operator
     delete op;
     return rc;
   }
@@ -735,6 +741,7 @@ extern "C" int gbpc_op_diagonal(int nrow, int block, const int32_t* offsets,
   }
   cudaError_t e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
+    tmp.release();
     delete op;
     gbpc_set_error_cuda(e, "diagonal setup", __FILE__, __LINE__);
     return GBPC_ERR_CUDA;
@@ -868,9 +875,14 @@ extern "C" int gbpc_op_bilu0(int nrow, int block, const int32_t* offsets, const 
   op->B = block;
   op->sweeps = solve_sweeps;
   DevBuf factors;
+  const size_t vec = vs * (size_t)std::max<int64_t>(op->rows, 1);
   int rc = factors.alloc(vs * std::max<int64_t>(nnz, 1) * bb);
-  if (!rc) rc = op->inv.alloc(vs * std::max<int64_t>((int64_t)nrow * bb, 1));
-  for (int k = 0; k < 4 && !rc; ++k) rc = op->buf[k].alloc(vs * std::max<int64_t>(op->rows, 1));
+  if (!rc)
+    rc = alloc_group(op->store, {{&op->inv, vs * std::max<int64_t>((int64_t)nrow * bb, 1)},
+                                 {&op->buf[0], vec},
+                                 {&op->buf[1], vec},
+                                 {&op->buf[2], vec},
+                                 {&op->buf[3], vec}});
   int32_t bad = 0;
   if (!rc)
     rc = bilu0_setup(nrow, block, offsets, columns, values, dtype, nnz, factor_sweeps, relaxation,
@@ -893,6 +905,7 @@ extern "C" int gbpc_op_bilu0(int nrow, int block, const int32_t* offsets, const 
   if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = GBPC_ERR_CUDA;
   if (rc) {
     if (rc == GBPC_ERR_CUDA) gbpc_set_error("gbpc_op_bilu0: CUDA failure");
+    factors.release();  // charged to the operator
     delete op;
     return rc;
   }

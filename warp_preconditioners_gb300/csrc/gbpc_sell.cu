@@ -107,10 +107,26 @@ int DevBuf::alloc(size_t n) {
   return GBPC_OK;
 }
 
-int ReduceBuf::init(cudaStream_t st) {
-  int rc = partials.alloc(sizeof(double) * kMaxCtas);
+int alloc_group(DevBuf& store, std::initializer_list<DevPart> parts) {
+  constexpr size_t kAlign = 256;
+  size_t total = 0;
+  for (const DevPart& q : parts) total += (q.bytes + kAlign - 1) / kAlign * kAlign;
+  int rc = store.alloc(total);
   if (rc) return rc;
-  rc = counter.alloc(sizeof(unsigned int));
+  char* at = store.as<char>();
+  for (const DevPart& q : parts) {
+    q.buf->release();
+    q.buf->p = at;
+    q.buf->bytes = q.bytes;
+    q.buf->part = true;
+    at += (q.bytes + kAlign - 1) / kAlign * kAlign;
+  }
+  return GBPC_OK;
+}
+
+int ReduceBuf::init(cudaStream_t st) {
+  int rc = alloc_group(store, {{&partials, sizeof(double) * kMaxCtas},
+                               {&counter, sizeof(unsigned int)}});
   if (rc) return rc;
   GBPC_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned int), st));
   return GBPC_OK;
@@ -437,20 +453,17 @@ int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const
   s.vdtype = out_dtype;
   s.nslices = (nrow_out + kSlice - 1) / kSlice;
   s.perm.release();
-  s.sched.release();
-  int rc = s.slice_ptr.alloc(sizeof(int64_t) * (s.nslices + 1));
-  if (rc) return rc;
-  DevBuf perm, widths, info;
+  int rc;
+  DevBuf temp, perm, widths, info, ptr, sched;
+  const size_t ns = (size_t)s.nslices;
   SellLayout h{};
-  if (s.nslices == 0) {
-    GBPC_CUDA_TRY(cudaMemsetAsync(s.slice_ptr.p, 0, sizeof(int64_t), st));
-  } else {
-    if ((rc = s.sched.alloc(sizeof(int4) * (size_t)s.nslices))) return rc;
-    if ((rc = s.err.alloc(sizeof(int32_t)))) return rc;
-    if ((rc = perm.alloc(sizeof(int32_t) * (size_t)nrow_out))) return rc;
-    if ((rc = widths.alloc(sizeof(int32_t) * 2 * (size_t)s.nslices))) return rc;
-    if ((rc = info.alloc(sizeof(SellLayout)))) return rc;
-    GBPC_CUDA_TRY(cudaMemsetAsync(s.err.p, 0, sizeof(int32_t), st));
+  if (s.nslices > 0) {
+    if ((rc = alloc_group(temp, {{&perm, sizeof(int32_t) * (size_t)nrow_out},
+                                 {&widths, sizeof(int32_t) * 2 * ns},
+                                 {&info, sizeof(SellLayout)},
+                                 {&ptr, sizeof(int64_t) * (ns + 1)},
+                                 {&sched, sizeof(int4) * ns}})))
+      return rc;
     int32_t* plain = widths.as<int32_t>();
     sell_layout_kernel<<<(nrow_out + kSortWindow - 1) / kSortWindow, kSortWindow, 0, st>>>(
         nrow_out, off, col, opt.rows, opt.colmap, opt.part, perm.as<int32_t>(), plain,
@@ -459,21 +472,34 @@ int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const
     GBPC_CUDA_TRY(cudaFuncSetAttribute(sell_schedule_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     sell_schedule_kernel<<<1, 1024, smem, st>>>(s.nslices, plain, plain + s.nslices,
-                                                s.slice_ptr.as<int64_t>(), s.sched.as<int4>(),
+                                                ptr.as<int64_t>(), sched.as<int4>(),
                                                 info.as<SellLayout>());
     GBPC_CUDA_TRY(cudaGetLastError());
     GBPC_CUDA_TRY(cudaMemcpyAsync(&h, info.p, sizeof(h), cudaMemcpyDeviceToHost, st));
     GBPC_CUDA_TRY(cudaStreamSynchronize(st));
-    if (h.sorted) {
-      std::swap(s.perm.p, perm.p);
-      std::swap(s.perm.bytes, perm.bytes);
-      std::swap(s.perm.tally, perm.tally);
-    }
-    if (h.widest >= kScheduleWidths && (rc = build_schedule(s, st))) return rc;
   }
   s.nent = h.nent;
-  if ((rc = s.cols.alloc(sizeof(int32_t) * s.nent))) return rc;
-  if ((rc = s.vals.alloc(dtype_size(out_dtype) * s.nent * B * B))) return rc;
+  if ((rc = alloc_group(s.store, {{&s.slice_ptr, sizeof(int64_t) * (ns + 1)},
+                                  {&s.sched, sizeof(int4) * ns},
+                                  {&s.err, sizeof(int32_t)},
+                                  {&s.misfit, sizeof(int32_t)},
+                                  {&s.perm, h.sorted ? sizeof(int32_t) * (size_t)nrow_out : 0},
+                                  {&s.cols, sizeof(int32_t) * s.nent},
+                                  {&s.vals, dtype_size(out_dtype) * s.nent * B * B}})))
+    return rc;
+  if (!h.sorted) s.perm.release();
+  GBPC_CUDA_TRY(cudaMemsetAsync(s.err.p, 0, sizeof(int32_t), st));
+  if (s.nslices == 0) {
+    GBPC_CUDA_TRY(cudaMemsetAsync(s.slice_ptr.p, 0, sizeof(int64_t), st));
+  } else {
+    if ((rc = vec_copy(s.slice_ptr.p, ptr.p, ptr.bytes, st))) return rc;
+    if (h.sorted && (rc = vec_copy(s.perm.p, perm.p, perm.bytes, st))) return rc;
+    if (h.widest >= kScheduleWidths) {
+      if ((rc = build_schedule(s, st))) return rc;
+    } else if ((rc = vec_copy(s.sched.p, sched.p, sched.bytes, st))) {
+      return rc;
+    }
+  }
   if (s.nslices > 0) {
     if (in_dtype == GBPC_BF16) {
       launch_fill<__nv_bfloat16, __nv_bfloat16>(s, B, off, col, val, opt, st);
@@ -517,9 +543,7 @@ int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val
     return GBPC_ERR_ARG;
   }
   if (s.nrow > 0) {
-    DevBuf bad;
-    int rc;
-    if ((rc = bad.alloc(sizeof(int32_t)))) return rc;
+    DevBuf& bad = s.misfit;
     GBPC_CUDA_TRY(cudaMemsetAsync(bad.p, 0, sizeof(int32_t), st));
     sell_fits_kernel<<<grid_for(s.nrow, kThreads), kThreads, 0, st>>>(
         s.nrow, off, col, opt.rows, opt.colmap, opt.part,
