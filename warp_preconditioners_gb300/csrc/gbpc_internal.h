@@ -105,7 +105,7 @@ struct Sell {
   DevBuf sched;      // int4[nslices]: product schedule, slices by width descending
   DevBuf err;        // int32[1]: set by a product kernel whose bounded wait gave up
   DevBuf misfit;     // int32[1]: rows that do not fit, counted by sell_refill
-  int variant = 0;   // product kernel variant chosen by sell_autotune
+  int variant = 0;   // product kernel (sell_choose_variant)
   int64_t nnz = 0;   // stored entries without padding
 };
 
@@ -127,11 +127,6 @@ int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val
 int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const int32_t* col,
                const void* val, int in_dtype, int out_dtype, const SellBuild& opt,
                cudaStream_t st);
-
-// Time the product kernel variants on `m` (vectors of dtype adtype) and keep
-// the fastest.  All variants sum each row in the same order, so the choice
-// never changes results.
-int sell_autotune(Sell& m, int adtype, cudaStream_t st);
 
 // Epilogues of the SELL product (see gbpc_sell.cu).
 enum EpiKind : int {

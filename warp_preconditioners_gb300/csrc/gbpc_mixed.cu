@@ -285,7 +285,6 @@ extern "C" int gbpc_op_matching_schur(int order, int n, const int32_t* k_off, co
     rc = (cudaMemcpyAsync(op->buf[6].p, mass, dtype_size(dtype) * n, cudaMemcpyDeviceToDevice,
                           st) == cudaSuccess) ? GBPC_OK : GBPC_ERR_CUDA;
   if (!rc) rc = sell_build(op->k, n, n, 1, k_off, k_col, k_val, dtype, dtype, SellBuild{}, st);
-  if (!rc) rc = sell_autotune(op->k, dtype, st);
   if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = GBPC_ERR_CUDA;
   if (rc) {
     delete op;

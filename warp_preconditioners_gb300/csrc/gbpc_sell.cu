@@ -435,6 +435,44 @@ static int build_schedule(Sell& s, cudaStream_t st) {
   return GBPC_OK;
 }
 
+// Product kernel variants (scalar rows; must match launch_variant in
+// gbpc_spmv.cuh).  All give the same results bit for bit, so the choice is a
+// rule on the block size and the number of slices:
+//   * scalar rows run the software-pipelined kernel (4), the fastest on every
+//     matrix measured, or within noise of it.  GB300, us a product, variants
+//     0 / 1 / 2 / 3 / 4, the matrix in rotation with two others:
+//       G of the 70^3 Q, width 8, float64        9.6 / 14.7 / 10.5 / 12.8 /  9.5
+//       its transpose                           14.3 / 17.1 / 14.9 / 17.8 / 13.5
+//       G, width 48                             37.6 / 36.6 / 39.7 / 47.1 / 35.6
+//       the same in bfloat16, float32 vectors   34.0 / 29.5 / 35.5 / 39.7 / 24.8
+//       in float32, float64 vectors             60.8 / 60.7 / 59.6 / 75.2 / 57.6
+//       Q itself (62 entries a row)             58.0 / 59.9 / 61.9 / 70.0 / 54.8
+//       7-point Laplacian, 63^3                  6.0 /  9.5 /  6.0 /  7.0 /  5.9
+//   * 3 x 3 blocks run the pipelined blocked kernel (4) once the slices fill a
+//     grid's warps (64^3 K (x) C: 33.1 us against 34.4), the one-slice kernel
+//     (0) below that, where both are launch latency;
+//   * other blocks run the one-slice kernel (2 x 2, 70^3 lifted system: 46.2
+//     us against 46.6).
+// Timing the variants at each build took 0.75 ms of launches, events and
+// allocations of a width-8 constructor at 70^3 and never chose otherwise.
+constexpr int kNumVariants = 6;
+constexpr int kPipelined = 4;
+
+static void choose_variant(Sell& m) {
+  // GBPC_SPMV_VARIANT=0..kNumVariants-1 fixes the variant (tests and
+  // tuning); blocked rows run variant 4 as the pipelined blocked kernel and
+  // the others as 0.
+  if (const char* e = std::getenv("GBPC_SPMV_VARIANT")) {
+    if (e[0] >= '0' && e[0] <= '9' && e[1] == '\0' && e[0] - '0' < kNumVariants) {
+      m.variant = m.nslices > 0 && m.B <= 3 ? e[0] - '0' : 0;
+      return;
+    }
+  }
+  if (m.B == 1) m.variant = kPipelined;
+  else if (m.B == 3 && m.nslices >= kSms * (kThreads / 32)) m.variant = kPipelined;
+  else m.variant = 0;
+}
+
 int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const int32_t* col,
                const void* val, int in_dtype, int out_dtype, const SellBuild& opt,
                cudaStream_t st) {
@@ -489,6 +527,7 @@ int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const
     return rc;
   if (!h.sorted) s.perm.release();
   GBPC_CUDA_TRY(cudaMemsetAsync(s.err.p, 0, sizeof(int32_t), st));
+  choose_variant(s);
   if (s.nslices == 0) {
     GBPC_CUDA_TRY(cudaMemsetAsync(s.slice_ptr.p, 0, sizeof(int64_t), st));
   } else {
@@ -606,86 +645,6 @@ int sell_spmv(const Sell& m, int adtype, const void* x, const void* y, void* z, 
     gbpc_set_error("vector dtype must be float64 or float32");
     return GBPC_ERR_ARG;
   }
-  if (rc) return rc;
-  GBPC_CUDA_TRY(cudaGetLastError());
-  return GBPC_OK;
-}
-
-// Kernel variants timed by the autotuner (scalar rows; must match
-// launch_variant in gbpc_spmv.cuh).
-constexpr int kNumVariants = 6;
-
-// The software-pipelined variant is the default: inside Krylov iterations
-// (matrix streamed from HBM, input vector warm) it was the fastest or within
-// 2 % on every product of the 70^3 biharmonic solve (forward and backward
-// factored operator, G, G^T).  Another variant replaces it only when it is
-// clearly faster (kSwitchMargin) in the timing below, as can happen on rows
-// much wider than these.
-constexpr int kDefaultVariant = 4;
-constexpr float kSwitchMargin = 0.90f;
-
-int sell_autotune(Sell& m, int adtype, cudaStream_t st) {
-  // Blocked rows: 2 x 2 and 3 x 3 blocks choose between the one-slice
-  // kernel (0) and the pipelined blocked kernel (4); other sizes run 0.
-  const bool blocked = m.B != 1;
-  if (m.nslices == 0 || m.B > 3) {
-    m.variant = 0;
-    return GBPC_OK;
-  }
-  // GBPC_SPMV_VARIANT=0..kNumVariants-1 fixes the variant (tests and
-  // tuning); every variant gives the same results.  Blocked rows run
-  // variant 4 as the pipelined blocked kernel and 1..3 as 0.
-  if (const char* e = std::getenv("GBPC_SPMV_VARIANT")) {
-    if (e[0] >= '0' && e[0] <= '9' && e[1] == '\0' && e[0] - '0' < kNumVariants) {
-      m.variant = e[0] - '0';
-      return GBPC_OK;
-    }
-  }
-  // Fewer slices than warps in one grid (kSms CTAs of kThreads): the
-  // product is launch-latency-bound and timing the variants measures noise,
-  // so the default stands without the timed launches.
-  if (m.nslices < kSms * (kThreads / 32)) {
-    m.variant = blocked ? 0 : kDefaultVariant;
-    return GBPC_OK;
-  }
-  const size_t vs = dtype_size(adtype);
-  DevBuf x, z;
-  int rc;
-  // Scalar lengths: nrow and ncol count B x B blocks.
-  const size_t xbytes = vs * (size_t)std::max(m.ncol, 1) * m.B;
-  const size_t zbytes = vs * (size_t)std::max(m.nrow, 1) * m.B;
-  if ((rc = x.alloc(xbytes))) return rc;
-  if ((rc = z.alloc(zbytes))) return rc;
-  GBPC_CUDA_TRY(cudaMemsetAsync(x.p, 0, xbytes, st));
-  cudaEvent_t e0, e1;
-  GBPC_CUDA_TRY(cudaEventCreate(&e0));
-  GBPC_CUDA_TRY(cudaEventCreate(&e1));
-  float ms[kNumVariants];
-  for (int v = 0; v < kNumVariants && !rc; ++v) {
-    ms[v] = 1e30f;
-    if (blocked && v != 0 && v != 4) continue;
-    if (v == 5) continue;  // the bulk-copy variant runs only when GBPC_SPMV_VARIANT=5 selects it
-    m.variant = v;
-    for (int w = 0; w < 2 && !rc; ++w)
-      rc = sell_spmv(m, adtype, x.p, nullptr, z.p, 1.0, 0.0, nullptr, EpiHost{}, nullptr, st);
-    cudaEventRecord(e0, st);
-    for (int w = 0; w < 5 && !rc; ++w)
-      rc = sell_spmv(m, adtype, x.p, nullptr, z.p, 1.0, 0.0, nullptr, EpiHost{}, nullptr, st);
-    cudaEventRecord(e1, st);
-    cudaEventSynchronize(e1);
-    ms[v] = 0.f;
-    cudaEventElapsedTime(&ms[v], e0, e1);
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  int best_v = kDefaultVariant;
-  if (blocked) {
-    best_v = ms[4] < ms[0] ? 4 : 0;
-  } else {
-    for (int v = 0; v < kNumVariants && !rc; ++v)
-      if (ms[v] < kSwitchMargin * ms[kDefaultVariant] && ms[v] < ms[best_v]) best_v = v;
-  }
-  m.variant = best_v;
   if (rc) return rc;
   GBPC_CUDA_TRY(cudaGetLastError());
   return GBPC_OK;
