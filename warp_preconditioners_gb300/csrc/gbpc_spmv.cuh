@@ -31,6 +31,27 @@ __device__ __forceinline__ A fma_t(A a, A b, A c);
 template <> __device__ __forceinline__ double fma_t<double>(double a, double b, double c) { return fma(a, b, c); }
 template <> __device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return fmaf(a, b, c); }
 
+// Widening a stored value to float64 on the integer pipes.  The conversion
+// instruction occupies the FP64 pipe as long as a multiply-add (~64 cycles a
+// warp), so a float32 factor applied to float64 vectors took 1.6 times as
+// long as a float64 one: 70^3 G, width 8 / 48 (GB300): 13.9 / 57.6 us a product with
+// it, 9.4 / 34.7 us without (float64 storage: 9.5 / 35.6).  Normal numbers and
+// zeros are re-biased bit for bit; the rest is converted.
+template <typename A, typename V>
+__device__ __forceinline__ A widen_value(V v) {
+  if constexpr (std::is_same<A, double>::value && !std::is_same<V, double>::value) {
+    const float f = to_float(v);
+    const uint32_t u = __float_as_uint(f), mag = u & 0x7fffffffu;
+    // 0x00800000 <= mag < 0x7f800000: a normal number.
+    if (mag - 0x00800000u < 0x7f000000u)
+      return __hiloint2double((int)((u & 0x80000000u) | ((mag >> 3) + 0x38000000u)), (int)(u << 29));
+    if (mag == 0) return __hiloint2double((int)u, 0);
+    return (double)f;
+  } else {
+    return widen<A, V>(v);
+  }
+}
+
 enum SpmvFlags : int { F_ALPHA_ZERO = 1, F_ALPHA_ONE = 2, F_BETA_ZERO = 4 };
 
 template <int B> struct Chunk { static constexpr int value = 8; };
@@ -155,7 +176,7 @@ sell_spmv_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A beta, i
 #pragma unroll
             for (int r = 0; r < B; ++r)
 #pragma unroll
-              for (int q = 0; q < B; ++q) acc[r] = fma_t<A>(widen<A, V>(vv[j][r * B + q]), xv[j][q], acc[r]);
+              for (int q = 0; q < B; ++q) acc[r] = fma_t<A>(widen_value<A, V>(vv[j][r * B + q]), xv[j][q], acc[r]);
           }
         }
       }
@@ -231,8 +252,8 @@ sell_spmv2_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A beta, 
         }
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
-          if (k0 + j < width1) acc1[0] = fma_t<A>(widen<A, V>(v1[j]), x1[j], acc1[0]);
-          if (k0 + j < width2) acc2[0] = fma_t<A>(widen<A, V>(v2[j]), x2[j], acc2[0]);
+          if (k0 + j < width1) acc1[0] = fma_t<A>(widen_value<A, V>(v1[j]), x1[j], acc1[0]);
+          if (k0 + j < width2) acc2[0] = fma_t<A>(widen_value<A, V>(v2[j]), x2[j], acc2[0]);
         }
       }
     }
@@ -332,7 +353,7 @@ sell_spmv_pipe_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A be
           for (int j = 0; j < CH; ++j) xv[j] = (c[j] >= 0) ? __ldg(x + c[j]) : A(0);
 #pragma unroll
           for (int j = 0; j < CH; ++j)
-            if (k0 + j < cur.width) acc[0] = fma_t<A>(widen<A, V>(v[j]), xv[j], acc[0]);
+            if (k0 + j < cur.width) acc[0] = fma_t<A>(widen_value<A, V>(v[j]), xv[j], acc[0]);
         }
       }
       spmv_finish<1, V, A, EPI, DOT>(m, cur.s * kSlice + lane, acc, y, z, alpha, beta, run,
@@ -439,7 +460,7 @@ sell_spmv_bpipe_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A b
               for (int r = 0; r < B; ++r)
 #pragma unroll
                 for (int q = 0; q < B; ++q)
-                  acc[r] = fma_t<A>(widen<A, V>(v[j][r * B + q]), xv[j][q], acc[r]);
+                  acc[r] = fma_t<A>(widen_value<A, V>(v[j][r * B + q]), xv[j][q], acc[r]);
             }
           }
         }
@@ -631,19 +652,19 @@ sell_spmv_bulk_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A be
     const V* sv = reinterpret_cast<const V*>(ring + (size_t)pst * Cfg::kStage + Cfg::kColBytes) +
                   lane;
     if (pn == 4) {
-      acc = fma_t<A>(widen<A, V>(sv[0]), px[0], acc);
-      acc = fma_t<A>(widen<A, V>(sv[kSlice]), px[1], acc);
-      acc = fma_t<A>(widen<A, V>(sv[2 * kSlice]), px[2], acc);
-      acc = fma_t<A>(widen<A, V>(sv[3 * kSlice]), px[3], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[0]), px[0], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[kSlice]), px[1], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[2 * kSlice]), px[2], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[3 * kSlice]), px[3], acc);
     } else if (pn == 3) {
-      acc = fma_t<A>(widen<A, V>(sv[0]), px[0], acc);
-      acc = fma_t<A>(widen<A, V>(sv[kSlice]), px[1], acc);
-      acc = fma_t<A>(widen<A, V>(sv[2 * kSlice]), px[2], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[0]), px[0], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[kSlice]), px[1], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[2 * kSlice]), px[2], acc);
     } else if (pn == 2) {
-      acc = fma_t<A>(widen<A, V>(sv[0]), px[0], acc);
-      acc = fma_t<A>(widen<A, V>(sv[kSlice]), px[1], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[0]), px[0], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[kSlice]), px[1], acc);
     } else {
-      acc = fma_t<A>(widen<A, V>(sv[0]), px[0], acc);
+      acc = fma_t<A>(widen_value<A, V>(sv[0]), px[0], acc);
     }
     if (plast) {
       A a1[1] = {acc};
@@ -730,7 +751,7 @@ sell_spmv_bulk_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A be
 // slices spread over the warps by a grid stride.
 // Every variant launches the same grid (one 1024-thread CTA per SM at most),
 // so the CTA partials of a fused dot product, and therefore its rounding, do
-// not depend on which variant the autotuner picked: results are identical
+// not depend on which variant runs: results are identical
 // whatever the timing (and whatever else shares the GPU).
 static int spmv_grid(int nslices, int /*minb*/) {
   const int warps_per_cta = kThreads / 32;
