@@ -36,3 +36,31 @@ def test_stored_values_widened_exactly(monkeypatch, variant, storage):
     op.apply(vec(np.ones(n)), None, z, 1.0, 0.0, cuda())
     # 0 + v * 1, then 0 + 1 * that: the value itself (zeros lose their sign).
     np.testing.assert_array_equal(z.cpu().numpy(), stored.to(torch.float64).numpy())
+
+
+@pytest.mark.parametrize("factor_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("side", [1, 5, 33, 90])
+def test_float32_apply_writes_float64(factor_dtype, side):
+    """The product that writes float64 itself gives the bits of the widening
+    kernel (alpha = 1, beta = 1 with y = 0), eagerly and in a captured graph."""
+    from warp_preconditioners_gb300 import FSAI, problems
+
+    a = problems.laplacian_2d(side) if side > 1 else ss.csr_matrix([[3.0]])
+    pre = FSAI(to_bsr(a), max_row_size=8, factor_dtype=factor_dtype, apply_dtype=torch.float32)
+    n = a.shape[0]
+    x = vec(np.random.default_rng(side).normal(size=n))
+    zeros, z1, z2 = torch.zeros_like(x), torch.empty_like(x), torch.empty_like(x)
+    pre.matvec(x, z1, z1, 1.0, 0.0)
+    pre.matvec(x, zeros, z2, 1.0, 1.0)
+    assert torch.equal(z1, z2)
+    xz = x.clone()
+    pre.matvec(xz, xz, xz, 1.0, 0.0)  # all three the same vector
+    assert torch.equal(xz, z1)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        pre.matvec(x, z2, z2, 1.0, 0.0)
+    z2.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(z1, z2)

@@ -47,11 +47,18 @@ struct ByteTally {
 // While open, kernels launched through launch_k on this thread carry the
 // programmatic dependent launch attribute (gbpc_common.cuh).
 struct PdlScope {
-  bool prev;
+  bool prev, prev_off;
   explicit PdlScope(bool on);
   ~PdlScope();
   PdlScope(const PdlScope&) = delete;
   PdlScope& operator=(const PdlScope&) = delete;
+};
+
+// Opened by an operator around its launches after the first one, whose
+// predecessor is its own kernel: the attribute, unless an enclosing
+// PdlScope(false) says no.
+struct PdlChain : PdlScope {
+  PdlChain();
 };
 
 // Owned device allocation, or (alloc_group) a part of another one.
@@ -136,6 +143,7 @@ enum EpiKind : int {
   EPI_TRI_LOWER = 3,  // z = aux0 - acc                      (aux0 = rhs); out2 = inv_block(aux1) z
   EPI_TRI_UPPER = 4,  // z = alpha * inv_block(aux1) * (aux0 - acc) + beta * y
                       //                            (aux0 = rhs, aux1 = inverse blocks)
+  EPI_WIDEN = 5,      // out2 = (double) acc; float32 vectors, alpha 1, beta 0
 };
 
 struct EpiHost {
@@ -190,6 +198,18 @@ struct Operator {
   // when zero.  `dot` (nullable) reduces dot(dot->w, z) in the final kernel.
   virtual int apply(const void* x, const void* y, void* z, double alpha, double beta,
                     const int* guard, const DotSpec* dot, cudaStream_t st) = 0;
+  // z = (double) (Op x) for an operator on float32 vectors, z float64, with
+  // the fused dot; false when the operator has no such path.
+  virtual bool apply_widened(const float* x, double* z, const int* guard, const DotSpec* dot,
+                             cudaStream_t st, int* rc) {
+    (void)x;
+    (void)z;
+    (void)guard;
+    (void)dot;
+    (void)st;
+    (void)rc;
+    return false;
+  }
   // True when x may not alias z in apply (the generic entry copies x first).
   virtual bool gathers_x() const { return true; }
   // The scalar float64 sliced-ELL matrices whose products in this order

@@ -694,7 +694,10 @@ struct Solver {
         rc = GBPC_ERR_CUDA;
         break;
       }
-      rc = record_init(b, x, cs);
+      {
+        PdlScope plain(false);
+        rc = record_init(b, x, cs);
+      }
       cudaGraph_t g2 = nullptr;
       cudaError_t e = cudaStreamEndCapture(cs, &g2);
       if (rc) break;

@@ -245,7 +245,20 @@ struct FsaiOp : Operator {
       rc = sell_spmv(g, vdtype, x, nullptr, tmp.p, 1.0, 0.0, guard, EpiHost{}, nullptr, st);
       if (rc) return rc;
     }
+    PdlChain chain;
     return sell_spmv(gt, vdtype, tmp.p, y, z, alpha, beta, guard, EpiHost{}, dot, st);
+  }
+  bool apply_widened(const float* x, double* z, const int* guard, const DotSpec* dot,
+                     cudaStream_t st, int* rc) override {
+    if (g.B != 1 || vdtype != GBPC_F32) return false;
+    *rc = sell_spmv(g, vdtype, x, nullptr, tmp.p, 1.0, 0.0, guard, EpiHost{}, nullptr, st);
+    if (*rc) return true;
+    PdlChain chain;
+    EpiHost e;
+    e.kind = EPI_WIDEN;
+    e.out2 = z;
+    *rc = sell_spmv(gt, vdtype, tmp.p, nullptr, nullptr, 1.0, 0.0, guard, e, dot, st);
+    return true;
   }
   bool gathers_x() const override { return false; }
   int scalar_products(const Sell** out, int max) const override {
@@ -291,6 +304,7 @@ struct SqlapOp : Operator {
       if (rc) return rc;
     }
     EpiHost b{EPI_SQLAP_BWD, wmass.p, x};
+    PdlChain chain;
     return sell_spmv(bwd, vdtype, tmp.p, y, z, alpha, beta, guard, b, dot, st);
   }
   bool gathers_x() const override { return false; }
@@ -391,6 +405,7 @@ struct Bilu0Op : Operator {
       if ((rc = sell_spmv(lower, vdtype, a, nullptr, out, 1.0, 0.0, guard, e, nullptr, st))) return rc;
       a = out;
     }
+    PdlChain chain;
     for (int s = 1; s < sweeps; ++s) {
       EpiHost e{EPI_TRI_UPPER, a, inv.p};
       const bool last = s == sweeps - 1;
@@ -415,10 +430,17 @@ int LowPrecisionOp::apply(const void* x, const void* y, void* z, double alpha, d
   // x is consumed into in32 before z is written, so x, y, z may alias.
   GBPC_CUDA_TRY(launch_k(narrow_kernel, g, kThreads, 0, st, rows, (const double*)x,
                          in32.as<float>(), guard));
-  int rc = inner->apply(in32.p, nullptr, out32.p, 1.0, 0.0, guard, nullptr, st);
+  // The launches after the first follow this operator's own kernels, and the
+  // last product writes the float64 result itself.  53^3 width-48 bfloat16
+  // factor (GB300), matrices from HBM: 37.2 us an apply with a widening kernel
+  // and full launch gaps, 30.8 us now.
+  PdlChain chain;
+  const bool unit = alpha == 1.0 && beta == 0.0;
+  int rc;
+  if (unit && inner->apply_widened(in32.as<float>(), (double*)z, guard, dot, st, &rc)) return rc;
+  rc = inner->apply(in32.p, nullptr, out32.p, 1.0, 0.0, guard, nullptr, st);
   if (rc) return rc;
   const Reduction red = make_reduction(dot);
-  const bool unit = alpha == 1.0 && beta == 0.0;
   if (unit)
     GBPC_CUDA_TRY(launch_k(widen_axpby_kernel<true>, g, kThreads, 0, st, rows,
                            (const float*)out32.as<float>(), (const double*)y, (double*)z, alpha,

@@ -68,6 +68,7 @@ namespace {
 std::atomic<size_t> g_live_bytes{0};
 thread_local size_t* t_tally = nullptr;
 thread_local bool t_pdl = false;
+thread_local bool t_pdl_off = false;  // inside a PdlScope(false)
 }  // namespace
 
 bool pdl_active() {
@@ -77,8 +78,15 @@ bool pdl_active() {
   }();
   return t_pdl && enabled;
 }
-PdlScope::PdlScope(bool on) : prev(t_pdl) { t_pdl = on; }
-PdlScope::~PdlScope() { t_pdl = prev; }
+PdlScope::PdlScope(bool on) : prev(t_pdl), prev_off(t_pdl_off) {
+  t_pdl = on;
+  t_pdl_off = !on;
+}
+PdlScope::~PdlScope() {
+  t_pdl = prev;
+  t_pdl_off = prev_off;
+}
+PdlChain::PdlChain() : PdlScope(!t_pdl_off) {}
 
 size_t* current_tally() { return t_tally; }
 size_t device_bytes_live() { return g_live_bytes.load(); }

@@ -23,7 +23,8 @@ template <typename A>
 struct EpiDev {
   const A* aux0;
   const A* aux1;
-  A* out2;  // EPI_TRI_LOWER: also receives inv_block(aux1) z (nullptr: none)
+  A* out2;  // EPI_TRI_LOWER: also receives inv_block(aux1) z (nullptr: none);
+            // EPI_WIDEN: the float64 output
 };
 
 template <typename A>
@@ -73,7 +74,9 @@ __device__ __forceinline__ void spmv_finish(const SellView<V>& m, int row, const
 #pragma unroll
     for (int r = 0; r < B; ++r) {
       const int64_t idx = (int64_t)orow * B + r;
-      if (EPI == EPI_AXPBY) {
+      if (EPI == EPI_WIDEN) {
+        out[r] = acc[r];
+      } else if (EPI == EPI_AXPBY) {
         A v = alpha_one ? acc[r] : alpha * acc[r];
         if (!beta_zero) v = fma_t<A>(beta, y[idx], v);
         out[r] = v;
@@ -114,7 +117,8 @@ __device__ __forceinline__ void spmv_finish(const SellView<V>& m, int row, const
 #pragma unroll
     for (int r = 0; r < B; ++r) {
       const int64_t idx = (int64_t)orow * B + r;
-      z[idx] = out[r];
+      if constexpr (EPI == EPI_WIDEN) reinterpret_cast<double*>(ep.out2)[idx] = (double)out[r];
+      else z[idx] = out[r];
       if (DOT) dot_part = fma((double)out[r], red.w[idx], dot_part);
     }
   }
@@ -906,6 +910,12 @@ static int dispatch_epi(const Sell& m, const void* x, const void* y, void* z, do
           launch_spmv<B, V, A, EPI_TRI_LOWER>(m, x, y, z, alpha, beta, guard, ep, red, st);
         else
           launch_spmv<B, V, A, EPI_TRI_UPPER>(m, x, y, z, alpha, beta, guard, ep, red, st);
+        return GBPC_OK;
+      }
+      break;
+    case EPI_WIDEN:
+      if constexpr (B == 1 && std::is_same<A, float>::value) {
+        launch_spmv<1, V, A, EPI_WIDEN>(m, x, y, z, 1.0, 0.0, guard, ep, red, st);
         return GBPC_OK;
       }
       break;
