@@ -146,6 +146,17 @@ int gbpc_fsai_refit(int n, const int32_t* a_off, const int32_t* a_col, const voi
                     double pivot_floor, void* out, int factor_dtype, int32_t* status_host,
                     void* stream);
 
+/* gbpc_fsai_refit for a matrix that has to have the topology (ref_off[n + 1],
+ * ref_col[nnz]) that the factor was built from: the two are compared on the
+ * device first, status_host[2] is set when they differ, and the refit then
+ * does nothing (its arrays are not read beyond that comparison; a_col holds
+ * nnz entries).  status_host[3]; one synchronisation for all of it. */
+int gbpc_fsai_refit_same(int n, const int32_t* a_off, const int32_t* a_col, const void* a_val,
+                         int dtype, const int32_t* ref_off, const int32_t* ref_col, int64_t nnz,
+                         const int32_t* g_off, const int32_t* g_col, int width,
+                         double pivot_floor, void* out, int factor_dtype, int32_t* status_host,
+                         void* stream);
+
 /* C = A diag(col_scale) B + diag(add_diag), float64 scalar CSR (col_scale,
  * add_diag nullable), on the device: the host SciPy assembly of the
  * smoothing operator Q = alpha M + K M^-1 K (results/dirichlet-tuning/

@@ -58,6 +58,8 @@ _SIGNATURES = {
     "gbpc_scalarize": [_int, _int, _vp, _vp, _vp, _int, _vp, _vp, _vp, _vp],
     "gbpc_convert_factor": [_int, _vp, _vp, _vp, _int, _vp, _int, _i32p, _vp],
     "gbpc_fsai_refit": [_int, _vp, _vp, _vp, _int, _vp, _vp, _int, _dbl, _vp, _int, _i32p, _vp],
+    "gbpc_fsai_refit_same": [_int, _vp, _vp, _vp, _int, _vp, _vp, ctypes.c_int64, _vp, _vp, _int,
+                             _dbl, _vp, _int, _i32p, _vp],
     "gbpc_transpose_map": [_int, _vp, _vp, _vp, _vp, _vp, _vp],
     "gbpc_spgemm": [_int, _int, _vp, _vp, _vp, _vp, _int, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                     _i64p, _vp],

@@ -71,7 +71,8 @@ __device__ __forceinline__ int lower_bound_row(const int32_t* col, int lo, int h
 template <typename T>
 __global__ void fsai_diag_kernel(int n, const int32_t* __restrict__ off,
                                  const int32_t* __restrict__ col, const T* __restrict__ val,
-                                 T* scale, int32_t* status) {
+                                 T* scale, int32_t* status, const int32_t* gate = nullptr) {
+  if (gate && *gate) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int lo = lower_bound_row(col, off[i], off[i + 1], i);
@@ -1258,7 +1259,8 @@ __global__ void __launch_bounds__(32 * kRefitWarps)
 fsai_refit_kernel(int n, const int32_t* __restrict__ a_off, const int32_t* __restrict__ a_col,
                   const T* __restrict__ a_val, const T* __restrict__ scale,
                   const int32_t* __restrict__ g_off, const int32_t* __restrict__ g_col, int width,
-                  T floor, S* out, int32_t* bad) {
+                  T floor, S* out, int32_t* bad, const int32_t* gate) {
+  if (gate && *gate) return;
   extern __shared__ __align__(16) unsigned char refit_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int row = blockIdx.x * kRefitWarps + w;
@@ -1349,7 +1351,8 @@ __global__ void __launch_bounds__(128)
 fsai_refit_row_kernel(int n, const int32_t* __restrict__ a_off, const int32_t* __restrict__ a_col,
                       const T* __restrict__ a_val, const T* __restrict__ scale,
                       const int32_t* __restrict__ g_off, const int32_t* __restrict__ g_col,
-                      T floor, S* out, int32_t* bad) {
+                      T floor, S* out, int32_t* bad, const int32_t* gate) {
+  if (gate && *gate) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int start = g_off[i];
@@ -1363,10 +1366,12 @@ fsai_refit_row_kernel(int n, const int32_t* __restrict__ a_off, const int32_t* _
   bool valid = true;
   for (int p = 0; p < size; ++p) {
     const int r = g_col[start + p];
-    const int rlo = a_off[r], rhi = a_off[r + 1];
+    const int rhi = a_off[r + 1];
+    int lo = a_off[r];
     for (int q = 0; q <= p; ++q) {
       const int c = g_col[start + q];
-      const int lo = lower_bound_row(a_col, rlo, rhi, c);
+      // The support is sorted: each search starts where the last one ended.
+      lo = lower_bound_row(a_col, lo, rhi, c);
       T a = T(0);
       if (lo < rhi && a_col[lo] == c) a = a_val[lo] * scale[r] * scale[c];
       for (int k = 0; k < q; ++k) a = a - chol[tri_index(p, k)] * chol[tri_index(q, k)];
@@ -1414,7 +1419,8 @@ fsai_refit_wide_kernel(int count, const int32_t* __restrict__ order, int64_t str
                        const int32_t* __restrict__ a_off, const int32_t* __restrict__ a_col,
                        const T* __restrict__ a_val, const T* __restrict__ scale,
                        const int32_t* __restrict__ g_off, const int32_t* __restrict__ g_col,
-                       int W, T floor, S* out, int32_t* bad) {
+                       int W, T floor, S* out, int32_t* bad, const int32_t* gate) {
+  if (gate && *gate) return;
   extern __shared__ __align__(16) unsigned char refit_wide_smem[];
   T* z = reinterpret_cast<T*>(refit_wide_smem) + threadIdx.x;  // z[p] at z[p * blockDim.x]
   const int nt = blockDim.x;
@@ -1997,26 +2003,73 @@ static bool refit_wide_enabled() {
   return on;
 }
 
+// Sets *differ when two topologies of n rows and nnz entries are not the
+// same.  WIDE: all arrays start on 16 bytes.  HBM-bound (70^3 Q: 174 MB).
+template <bool WIDE>
+__global__ void __launch_bounds__(256)
+same_topology_kernel(int64_t n1, int64_t nnz, const int32_t* __restrict__ off_a,
+                     const int32_t* __restrict__ off_b, const int32_t* __restrict__ col_a,
+                     const int32_t* __restrict__ col_b, int32_t* differ) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  bool same = true;
+  for (int64_t i = t; i < n1; i += step) same = same && off_a[i] == off_b[i];
+  int64_t done = 0;
+  if (WIDE) {
+    const int4* a4 = reinterpret_cast<const int4*>(col_a);
+    const int4* b4 = reinterpret_cast<const int4*>(col_b);
+    for (int64_t i = t; i < nnz / 4; i += step) {
+      const int4 a = a4[i], b = b4[i];
+      same = same && a.x == b.x && a.y == b.y && a.z == b.z && a.w == b.w;
+    }
+    done = nnz / 4 * 4;
+  }
+  for (int64_t i = done + t; i < nnz; i += step) same = same && col_a[i] == col_b[i];
+  if (!same) *differ = 1;
+}
+
+// The topology a refit must find: when `off` is given, the matrix is compared
+// with it first, on the device, and the other kernels do nothing unless it is
+// the same, so the host reads one set of flags at the end.
+struct RefitTopology {
+  const int32_t* off = nullptr;
+  const int32_t* col = nullptr;
+  int64_t nnz = 0;
+};
+
+// status_host: rows with an invalid diagonal, invalid rows, topology differs.
 template <typename T, typename S>
 static int refit_t(int n, const int32_t* a_off, const int32_t* a_col, const T* a_val,
-                   const int32_t* g_off, const int32_t* g_col, int width, double floor_, S* out,
-                   int32_t* status_host, cudaStream_t st) {
+                   const RefitTopology& ref, const int32_t* g_off, const int32_t* g_col, int width,
+                   double floor_, S* out, int32_t* status_host, cudaStream_t st) {
   DevBuf work, scale, status;
   int rc;
   if ((rc = alloc_group(work, {{&scale, sizeof(T) * std::max(n, 1)},
-                               {&status, sizeof(int32_t) * 2}})))
+                               {&status, sizeof(int32_t) * 3}})))
     return rc;
-  GBPC_CUDA_TRY(cudaMemsetAsync(status.p, 0, sizeof(int32_t) * 2, st));
+  GBPC_CUDA_TRY(cudaMemsetAsync(status.p, 0, sizeof(int32_t) * 3, st));
   int32_t* stat = status.as<int32_t>();
+  const int32_t* gate = nullptr;
+  if (n > 0 && ref.off) {
+    gate = stat + 2;
+    const uintptr_t bits = (uintptr_t)a_col | (uintptr_t)ref.col;
+    const int g = (int)std::min<int64_t>((std::max<int64_t>(ref.nnz / 4, n) + 256) / 256, 152 * 8);
+    if (bits % 16 == 0)
+      same_topology_kernel<true><<<g, 256, 0, st>>>((int64_t)n + 1, ref.nnz, a_off, ref.off, a_col,
+                                                    ref.col, stat + 2);
+    else
+      same_topology_kernel<false><<<g, 256, 0, st>>>((int64_t)n + 1, ref.nnz, a_off, ref.off,
+                                                     a_col, ref.col, stat + 2);
+  }
   if (n > 0) {
     fsai_diag_kernel<T><<<grid_for(n, 256), 256, 0, st>>>(n, a_off, a_col, a_val, scale.as<T>(),
-                                                          stat);
+                                                          stat, gate);
     if (width <= 8) {
       fsai_refit_row_kernel<T, S, 8><<<grid_for(n, 128), 128, 0, st>>>(
-          n, a_off, a_col, a_val, scale.as<T>(), g_off, g_col, (T)floor_, out, stat + 1);
+          n, a_off, a_col, a_val, scale.as<T>(), g_off, g_col, (T)floor_, out, stat + 1, gate);
     } else if (width <= 16) {
       fsai_refit_row_kernel<T, S, 16><<<grid_for(n, 128), 128, 0, st>>>(
-          n, a_off, a_col, a_val, scale.as<T>(), g_off, g_col, (T)floor_, out, stat + 1);
+          n, a_off, a_col, a_val, scale.as<T>(), g_off, g_col, (T)floor_, out, stat + 1, gate);
     } else if (refit_wide_enabled()) {
       // Thread per row, rows in order of support size, the local factors of
       // a chunk of rows in device memory (a quarter of the free memory, 8 GB
@@ -2047,7 +2100,7 @@ static int refit_t(int n, const int32_t* a_off, const int32_t* a_col, const T* a
         const int cnt = std::min(nc, n - k0);
         fsai_refit_wide_kernel<T, S><<<grid_for(cnt, ft), ft, smem, st>>>(
             cnt, order.as<int32_t>() + k0, (int64_t)cnt, lbuf.as<T>(), a_off, a_col, a_val,
-            scale.as<T>(), g_off, g_col, width, (T)floor_, out, stat + 1);
+            scale.as<T>(), g_off, g_col, width, (T)floor_, out, stat + 1, gate);
       }
     } else {
       const size_t smem = sizeof(T) * (size_t)(width * (width + 1) / 2 + width) * kRefitWarps;
@@ -2055,20 +2108,20 @@ static int refit_t(int n, const int32_t* a_off, const int32_t* a_col, const T* a
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       fsai_refit_kernel<T, S><<<(n + kRefitWarps - 1) / kRefitWarps, 32 * kRefitWarps, smem,
                                 st>>>(n, a_off, a_col, a_val, scale.as<T>(), g_off, g_col, width,
-                                      (T)floor_, out, stat + 1);
+                                      (T)floor_, out, stat + 1, gate);
     }
   }
   GBPC_CUDA_TRY(cudaGetLastError());
-  GBPC_CUDA_TRY(cudaMemcpyAsync(status_host, stat, sizeof(int32_t) * 2, cudaMemcpyDeviceToHost, st));
+  GBPC_CUDA_TRY(cudaMemcpyAsync(status_host, stat, sizeof(int32_t) * 3, cudaMemcpyDeviceToHost, st));
   GBPC_CUDA_TRY(cudaStreamSynchronize(st));
   return GBPC_OK;
 }
 }  // namespace gbpc
 
-extern "C" int gbpc_fsai_refit(int n, const int32_t* a_off, const int32_t* a_col,
-                               const void* a_val, int dtype, const int32_t* g_off,
-                               const int32_t* g_col, int width, double pivot_floor, void* out,
-                               int factor_dtype, int32_t* status_host, void* stream) {
+static int refit_any(int n, const int32_t* a_off, const int32_t* a_col, const void* a_val,
+                     int dtype, const RefitTopology& ref, const int32_t* g_off,
+                     const int32_t* g_col, int width, double pivot_floor, void* out,
+                     int factor_dtype, int32_t* status_host, void* stream) {
   NvtxRange nvtx_range("gbpc_fsai_refit");
   if (n < 0 || width < 1 || width > 64 || !status_host ||
       (n > 0 && (!a_off || !a_col || !a_val || !g_off || !g_col || !out)) ||
@@ -2079,27 +2132,54 @@ extern "C" int gbpc_fsai_refit(int n, const int32_t* a_off, const int32_t* a_col
   cudaStream_t st = (cudaStream_t)stream;
   if (dtype == GBPC_F64) {
     if (factor_dtype == GBPC_F64)
-      return refit_t<double, double>(n, a_off, a_col, (const double*)a_val, g_off, g_col, width,
+      return refit_t<double, double>(n, a_off, a_col, (const double*)a_val, ref, g_off, g_col, width,
                                      pivot_floor, (double*)out, status_host, st);
     if (factor_dtype == GBPC_F32)
-      return refit_t<double, float>(n, a_off, a_col, (const double*)a_val, g_off, g_col, width,
+      return refit_t<double, float>(n, a_off, a_col, (const double*)a_val, ref, g_off, g_col, width,
                                     pivot_floor, (float*)out, status_host, st);
     if (factor_dtype == GBPC_BF16)
-      return refit_t<double, __nv_bfloat16>(n, a_off, a_col, (const double*)a_val, g_off, g_col,
+      return refit_t<double, __nv_bfloat16>(n, a_off, a_col, (const double*)a_val, ref, g_off, g_col,
                                             width, pivot_floor, (__nv_bfloat16*)out, status_host,
                                             st);
   } else if (dtype == GBPC_F32) {
     if (factor_dtype == GBPC_F32)
-      return refit_t<float, float>(n, a_off, a_col, (const float*)a_val, g_off, g_col, width,
+      return refit_t<float, float>(n, a_off, a_col, (const float*)a_val, ref, g_off, g_col, width,
                                    pivot_floor, (float*)out, status_host, st);
     if (factor_dtype == GBPC_BF16)
-      return refit_t<float, __nv_bfloat16>(n, a_off, a_col, (const float*)a_val, g_off, g_col,
+      return refit_t<float, __nv_bfloat16>(n, a_off, a_col, (const float*)a_val, ref, g_off, g_col,
                                            width, pivot_floor, (__nv_bfloat16*)out, status_host,
                                            st);
   }
   gbpc_set_error("gbpc_fsai_refit: unsupported matrix / factor dtype pair (%d, %d)", dtype,
                  factor_dtype);
   return GBPC_ERR_ARG;
+}
+
+extern "C" int gbpc_fsai_refit(int n, const int32_t* a_off, const int32_t* a_col,
+                               const void* a_val, int dtype, const int32_t* g_off,
+                               const int32_t* g_col, int width, double pivot_floor, void* out,
+                               int factor_dtype, int32_t* status_host, void* stream) {
+  int32_t status[3] = {0, 0, 0};
+  const int rc = refit_any(n, a_off, a_col, a_val, dtype, RefitTopology{}, g_off, g_col, width,
+                           pivot_floor, out, factor_dtype, status_host ? status : nullptr, stream);
+  if (!rc) {
+    status_host[0] = status[0];
+    status_host[1] = status[1];
+  }
+  return rc;
+}
+
+extern "C" int gbpc_fsai_refit_same(int n, const int32_t* a_off, const int32_t* a_col,
+                                    const void* a_val, int dtype, const int32_t* ref_off,
+                                    const int32_t* ref_col, int64_t nnz, const int32_t* g_off,
+                                    const int32_t* g_col, int width, double pivot_floor, void* out,
+                                    int factor_dtype, int32_t* status_host, void* stream) {
+  if (n > 0 && (!ref_off || (nnz > 0 && !ref_col) || nnz < 0)) {
+    gbpc_set_error("gbpc_fsai_refit_same: bad arguments");
+    return GBPC_ERR_ARG;
+  }
+  return refit_any(n, a_off, a_col, a_val, dtype, RefitTopology{ref_off, ref_col, nnz}, g_off,
+                   g_col, width, pivot_floor, out, factor_dtype, status_host, stream);
 }
 
 extern "C" int gbpc_transpose_map(int nrow, const int32_t* offsets, const int32_t* columns,

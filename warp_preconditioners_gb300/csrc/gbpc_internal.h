@@ -111,7 +111,7 @@ struct Sell {
   DevBuf perm;       // int32[nrow] when rows are stored sorted by length
   DevBuf sched;      // int4[nslices]: product schedule, slices by width descending
   DevBuf err;        // int32[1]: set by a product kernel whose bounded wait gave up
-  DevBuf misfit;     // int32[1]: rows that do not fit, counted by sell_refill
+  DevBuf misfit;     // int32[1]: rows that do not fit, counted by sell_count_misfits
   int variant = 0;   // product kernel (sell_choose_variant)
   int64_t nnz = 0;   // stored entries without padding
 };
@@ -128,7 +128,10 @@ struct SellBuild {
   const void* row_scale = nullptr;  // optional per-source-row factor (input value dtype)
 };
 
-// Rewrites the values of a Sell built from the same pattern (off, col, opt).
+// Rewrites the values of a Sell built from the same pattern (off, col, opt);
+// only for a pattern without rows that do not fit, which the other counts.
+int sell_count_misfits(Sell& s, const int32_t* off, const int32_t* col, int in_dtype,
+                       const SellBuild& opt, int32_t* misfit_host, cudaStream_t st);
 int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val, int in_dtype,
                 const SellBuild& opt, cudaStream_t st);
 int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const int32_t* col,

@@ -598,8 +598,20 @@ extern "C" int gbpc_op_fsai_refill(gbpc_op* h, const int32_t* g_off, const int32
   }
   cudaStream_t st = (cudaStream_t)stream;
   const int in = input_dtype(value_dtype);
-  int rc = sell_refill(op->g, g_off, g_col, g_val, in, SellBuild{}, st);
-  if (!rc) rc = sell_refill(op->gt, gt_off, gt_col, gt_val, in, SellBuild{}, st);
+  // Both patterns are checked before either matrix changes, with one wait.
+  const SellBuild all{};
+  int32_t misfits[2] = {0, 0};
+  int rc = sell_count_misfits(op->g, g_off, g_col, in, all, misfits, st);
+  if (!rc) rc = sell_count_misfits(op->gt, gt_off, gt_col, in, all, misfits + 1, st);
+  if (rc) return rc;
+  GBPC_CUDA_TRY(cudaStreamSynchronize(st));
+  if (misfits[0] || misfits[1]) {
+    gbpc_set_error("refill: %d rows do not fit the operator's layout (pattern changed)",
+                   misfits[0] ? misfits[0] : misfits[1]);
+    return GBPC_ERR_ARG;
+  }
+  rc = sell_refill(op->g, g_off, g_col, g_val, in, all, st);
+  if (!rc) rc = sell_refill(op->gt, gt_off, gt_col, gt_val, in, all, st);
   return rc;
 }
 

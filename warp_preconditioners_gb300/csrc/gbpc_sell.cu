@@ -579,12 +579,12 @@ __global__ void sell_fits_kernel(int nrow, const int32_t* __restrict__ off,
   if (row_length(r, off, col, rows, colmap, part) > width) atomicAdd(bad, 1);
 }
 
-// New values for an unchanged pattern: the fill pass again over the existing
-// layout (slices, row order, columns), writing vals in place, so captured
-// products see them.  Rejects a pattern whose rows do not fit the layout.
-int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val, int in_dtype,
-                const SellBuild& opt, cudaStream_t st) {
+// Counts the rows of a pattern that do not fit the layout into *misfit_host
+// (stream-ordered).
+int sell_count_misfits(Sell& s, const int32_t* off, const int32_t* col, int in_dtype,
+                       const SellBuild& opt, int32_t* misfit_host, cudaStream_t st) {
   const int out_dtype = s.vdtype;
+  *misfit_host = 0;
   if (!valid_value_dtype(in_dtype) || (in_dtype == GBPC_BF16 && out_dtype != GBPC_BF16)) {
     gbpc_set_error("unsupported value dtype %d -> %d", in_dtype, out_dtype);
     return GBPC_ERR_ARG;
@@ -597,14 +597,17 @@ int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val
         s.perm.p ? s.perm.as<int32_t>() : nullptr,
         s.slice_ptr.as<int64_t>(), bad.as<int32_t>());
     GBPC_CUDA_TRY(cudaGetLastError());
-    int32_t h = 0;
-    GBPC_CUDA_TRY(cudaMemcpyAsync(&h, bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GBPC_CUDA_TRY(cudaStreamSynchronize(st));
-    if (h) {
-      gbpc_set_error("refill: %d rows do not fit the operator's layout (pattern changed)", h);
-      return GBPC_ERR_ARG;
-    }
+    GBPC_CUDA_TRY(cudaMemcpyAsync(misfit_host, bad.p, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
   }
+  return GBPC_OK;
+}
+
+// New values for an unchanged pattern: the fill pass again over the existing
+// layout (slices, row order, columns), writing vals in place, so captured
+// products see them.
+int sell_refill(Sell& s, const int32_t* off, const int32_t* col, const void* val, int in_dtype,
+                const SellBuild& opt, cudaStream_t st) {
+  const int out_dtype = s.vdtype;
   if (s.nslices > 0) {
     if (in_dtype == GBPC_BF16) {
       launch_fill<__nv_bfloat16, __nv_bfloat16>(s, s.B, off, col, val, opt, st);

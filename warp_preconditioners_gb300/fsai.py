@@ -247,20 +247,34 @@ class _RefitPlan:
             raise ValueError("FSAI update requires the original shape, dtype, device and topology")
         if A.offsets.shape != self.offsets.shape or A.columns.shape != self.columns.shape:
             raise ValueError("FSAI update requires identical topology storage")
-        if not (torch.equal(A.offsets, self.offsets) and torch.equal(A.columns, self.columns)):
-            raise ValueError("FSAI update requires identical sparsity; rebuild to change it")
-        if A.values.numel() < self.columns.numel() * A.block_size:
-            raise ValueError("Insufficient source values")
         G, GT = owner.G, owner.GT
+        enough = A.values.numel() >= self.columns.numel() * A.block_size
+        # A scalar matrix is compared with the topology in the refit itself
+        # (one wait for its flags); a blocked one before it is scalarised.
+        fused = (A.block_size == 1 and enough and G.nrow > 0
+                 and A.offsets.dtype == torch.int32 and A.columns.dtype == torch.int32
+                 and A.offsets.is_contiguous() and A.columns.is_contiguous())
+        if not fused and not (torch.equal(A.offsets, self.offsets)
+                              and torch.equal(A.columns, self.columns)):
+            raise ValueError("FSAI update requires identical sparsity; rebuild to change it")
+        if not enough:
+            raise ValueError("Insufficient source values")
         if G.nrow == 0:
             return
         scalar = scalarize(A)
         st = _lib.stream(A.device)
-        status = (ctypes.c_int32 * 2)()
-        _lib.call("gbpc_fsai_refit", G.nrow, _lib.ptr(scalar.offsets), _lib.ptr(scalar.columns),
-                  _lib.ptr(scalar.values.reshape(-1)), _lib.dtype_code(scalar.scalar_type),
-                  _lib.ptr(G.offsets), _lib.ptr(G.columns), self.width, self.floor,
-                  _lib.ptr(self.candidate), _lib.dtype_code(G.scalar_type), status, st)
+        status = (ctypes.c_int32 * 3)()
+        args = [G.nrow, _lib.ptr(scalar.offsets), _lib.ptr(scalar.columns),
+                _lib.ptr(scalar.values.reshape(-1)), _lib.dtype_code(scalar.scalar_type)]
+        rest = [_lib.ptr(G.offsets), _lib.ptr(G.columns), self.width, self.floor,
+                _lib.ptr(self.candidate), _lib.dtype_code(G.scalar_type), status, st]
+        if fused:
+            _lib.call("gbpc_fsai_refit_same", *args, _lib.ptr(self.offsets),
+                      _lib.ptr(self.columns), int(self.columns.numel()), *rest)
+        else:
+            _lib.call("gbpc_fsai_refit", *args, *rest)
+        if status[2]:
+            raise ValueError("FSAI update requires identical sparsity; rebuild to change it")
         if status[0] or status[1]:
             raise ValueError("FSAI refit requires finite positive diagonals and SPD local supports")
         G.values.copy_(self.candidate)
