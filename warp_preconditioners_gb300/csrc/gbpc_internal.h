@@ -104,6 +104,7 @@ struct Sell {
   int nslices = 0;
   int vdtype = GBPC_F64;
   int64_t nent = 0;  // entries including padding
+  int widest = 0;    // at least the width of every slice
   DevBuf slice_ptr;  // int64[nslices + 1]
   DevBuf cols;       // int32[nent]
   DevBuf vals;       // vdtype[nent * B * B]

@@ -210,11 +210,21 @@ struct Args {
   double* x;
   double *r, *z, *p, *Ap, *t, *u;
   KrylovScalars* ks;
+  // smax > 0: the system fits the cluster's shared memory (pcg_resident);
+  // the most slices a CTA owns and the widths of A, G and GT.
+  int smax;
+  int wide[3];
 };
 
 // Row epilogues of `product`, those of the sliced-ELL kernels: plain,
 // (1/m) o acc, acc + (w m) o x.
 enum CoopEpi : int { CE_PLAIN = 0, CE_SCALE = 1, CE_MASS = 2 };
+
+// First slice of CTA c of a cluster: a CTA owns consecutive slices, and the
+// rows of every vector that they hold in the plain row order.
+__host__ __device__ __forceinline__ int cluster_slice(int nslices, int cta, int ncta) {
+  return (int)((int64_t)nslices * cta / ncta);
+}
 
 // z = m x (one warp per slice, rows in storage order); dot_part += z . w.
 __device__ __forceinline__ void product(const Mat& m, const double* x, double* z, const double* w,
@@ -222,8 +232,9 @@ __device__ __forceinline__ void product(const Mat& m, const double* x, double* z
                                         int epi = CE_PLAIN, const double* aux0 = nullptr,
                                         const double* aux1 = nullptr) {
   const int lane = threadIdx.x & 31;
-  const int nwarps = ncta * (kThreadsC / 32);
-  for (int s = cta * (kThreadsC / 32) + (threadIdx.x >> 5); s < m.nslices; s += nwarps) {
+  const int end = cluster_slice(m.nslices, cta + 1, ncta);
+  for (int s = cluster_slice(m.nslices, cta, ncta) + (threadIdx.x >> 5); s < end;
+       s += kThreadsC / 32) {
     const int64_t base = m.slice_ptr[s];
     const int width = (int)((m.slice_ptr[s + 1] - base) / kSlice);
     double acc = 0.0;
@@ -258,21 +269,8 @@ __device__ __forceinline__ void product(const Mat& m, const double* x, double* z
   }
 }
 
-// CTA sum of one value per thread, in thread 0 (fixed order).
-__device__ __forceinline__ double cta_sum(double v, double* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  double c = 0.0;
-  if (threadIdx.x == 0)
-    for (int w2 = 0; w2 < kThreadsC / 32; ++w2) c += sh[w2];
-  return c;
-}
-
-// Synchronisation and the exchange of per-CTA sums.  Every CTA gets the
-// same total: the CTA sums added in CTA order (lanes take them strided,
+// Synchronisation and the exchange of per-warp sums.  Every CTA gets the
+// same total: the warp sums added in warp order (lanes take them strided,
 // then a fixed butterfly).  Two slots alternate, so a CTA that runs ahead
 // never overwrites sums another CTA is still reading.
 //
@@ -281,24 +279,27 @@ __device__ __forceinline__ double cta_sum(double v, double* sh) {
 // their shared memory (distributed shared memory), no global round trip.
 struct ClusterSync {
   cgr::cluster_group c;
-  double* xch;  // this CTA's shared [2] exchange slots
+  double* xch;  // this CTA's shared [2][warps] exchange slots
   __device__ ClusterSync(double* x) : c(cgr::this_cluster()), xch(x) {}
   __device__ void sync() { c.sync(); }
   __device__ double total(double v, int slot, double* sh) {
+    constexpr int kWarps = kThreadsC / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double cs = cta_sum(v, sh);
-    if (threadIdx.x == 0) xch[slot] = cs;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) xch[slot * kWarps + warp] = v;
     c.sync();
     if (warp == 0) {
-      const unsigned int ranks = c.num_blocks();
+      const int parts = (int)c.num_blocks() * kWarps;
       double a = 0.0;
-      for (unsigned int q = lane; q < ranks; q += 32) a += *c.map_shared_rank(xch + slot, q);
+      for (int q = lane; q < parts; q += 32)
+        a += *c.map_shared_rank(xch + slot * kWarps + q % kWarps, q / kWarps);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-      if (lane == 0) sh[kThreadsC / 32] = a;
+      if (lane == 0) *sh = a;
     }
     __syncthreads();
-    const double t = sh[kThreadsC / 32];
+    const double t = *sh;
     __syncthreads();
     return t;
   }
@@ -324,8 +325,8 @@ __device__ __forceinline__ void apply_a(S& grid, const Args& a, const double* x,
 // z = M r (G then G^T, a sync between them; or z = r); returns this
 // thread's share of r.z.
 template <class S>
-__device__ __forceinline__ double precondition(S& grid, const Args& a, bool precond, int64_t gt,
-                                               int64_t gs, int cta, int ncta) {
+__device__ __forceinline__ double precondition(S& grid, const Args& a, bool precond, int64_t i0,
+                                               int64_t i1, int cta, int ncta) {
   double prz = 0.0;
   if (precond) {
     double d0 = 0.0;
@@ -333,7 +334,7 @@ __device__ __forceinline__ double precondition(S& grid, const Args& a, bool prec
     grid.sync();
     product(a.GT, a.t, a.z, a.r, prz, cta, ncta);
   } else {
-    for (int64_t i = gt; i < a.n; i += gs) {
+    for (int64_t i = i0; i < i1; i += kThreadsC) {
       const double ri = a.r[i];
       a.z[i] = ri;
       prz = fma(ri, ri, prz);
@@ -347,8 +348,11 @@ template <class S>
 __device__ void pcg_body(const Args& a, S& grid, int cta, int ncta, double* sh) {
   KrylovScalars* ks = a.ks;
   const int64_t n = a.n;
-  const int64_t gt = (int64_t)cta * kThreadsC + threadIdx.x;
-  const int64_t gs = (int64_t)ncta * kThreadsC;
+  // This thread's rows: i0, i0 + kThreadsC, ... below i1.
+  const int nslices = a.A.nslices;
+  const int64_t i0 = (int64_t)cluster_slice(nslices, cta, ncta) * kSlice + threadIdx.x;
+  const int64_t i1 = min(n, (int64_t)cluster_slice(nslices, cta + 1, ncta) * kSlice);
+  const bool first_thread = cta == 0 && threadIdx.x == 0;
   const bool precond = a.G.nslices >= 0;
   int slot = 0;
   const double tol = ks->tol, atol = ks->atol;
@@ -360,7 +364,7 @@ __device__ void pcg_body(const Args& a, S& grid, int cta, int ncta, double* sh) 
   apply_a(grid, a, a.x, a.Ap, nullptr, dummy, cta, ncta);
   grid.sync();
   double pbb = 0.0, prr = 0.0;
-  for (int64_t i = gt; i < n; i += gs) {
+  for (int64_t i = i0; i < i1; i += kThreadsC) {
     const double bi = a.b[i];
     const double ri = bi - a.Ap[i];
     a.r[i] = ri;
@@ -373,12 +377,12 @@ __device__ void pcg_body(const Args& a, S& grid, int cta, int ncta, double* sh) 
   slot ^= 1;
   const double at = fmax(atol, tol * sqrt(bb));
   const double atol_sq = at * at;
-  if (gt == 0 && hist && hist_len > 0) hist[0] = sqrt(rr);
+  if (first_thread && hist && hist_len > 0) hist[0] = sqrt(rr);
   // z = M r, rz = r.z, p = z.
-  double prz = precondition(grid, a, precond, gt, gs, cta, ncta);
+  double prz = precondition(grid, a, precond, i0, i1, cta, ncta);
   double rz = grid.total(prz, slot, sh);
   slot ^= 1;
-  for (int64_t i = gt; i < n; i += gs) a.p[i] = a.z[i];
+  for (int64_t i = i0; i < i1; i += kThreadsC) a.p[i] = a.z[i];
   grid.sync();
   int it = 0;
   double alpha = 0.0, beta = 0.0, pap = 0.0;
@@ -389,7 +393,7 @@ __device__ void pcg_body(const Args& a, S& grid, int cta, int ncta, double* sh) 
     slot ^= 1;
     alpha = rz / pap;
     double prr2 = 0.0;
-    for (int64_t i = gt; i < n; i += gs) {
+    for (int64_t i = i0; i < i1; i += kThreadsC) {
       a.x[i] = fma(alpha, a.p[i], a.x[i]);
       const double ri = fma(-alpha, a.Ap[i], a.r[i]);
       a.r[i] = ri;
@@ -397,18 +401,297 @@ __device__ void pcg_body(const Args& a, S& grid, int cta, int ncta, double* sh) 
     }
     rr = grid.total(prr2, slot, sh);
     slot ^= 1;
-    if (gt == 0 && hist && it + 1 < hist_len) hist[it + 1] = sqrt(rr);
-    const double prz2 = precondition(grid, a, precond, gt, gs, cta, ncta);
+    if (first_thread && hist && it + 1 < hist_len) hist[it + 1] = sqrt(rr);
+    const double prz2 = precondition(grid, a, precond, i0, i1, cta, ncta);
     const double rz_new = grid.total(prz2, slot, sh);
     slot ^= 1;
     beta = rz_new / rz;
     rz = rz_new;
     ++it;
-    for (int64_t i = gt; i < n; i += gs) a.p[i] = fma(beta, a.p[i], a.z[i]);
+    for (int64_t i = i0; i < i1; i += kThreadsC) a.p[i] = fma(beta, a.p[i], a.z[i]);
     grid.sync();
   }
   grid.finish();
-  if (gt == 0) {
+  if (first_thread) {
+    ks->bb = bb;
+    ks->atol_sq = atol_sq;
+    ks->rr = rr;
+    ks->rz = rz;
+    ks->denom = pap;
+    ks->alpha = alpha;
+    ks->beta = beta;
+    ks->it = it;
+    ks->active = 0;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same solve with everything in the cluster's shared memory.
+//
+// pcg_body's phases are short (one slice a warp and matrix at 4,096 rows) and
+// bound by latency: every cluster barrier empties the L1, so each phase read
+// its matrix and its vectors from L2 again, one round trip after the other,
+// and each of the three totals chained ten FP64 adds, two block barriers and
+// a read of the other CTAs' sums; every thread did alpha's division.  Here a
+// CTA keeps its slices of A, G and GT and its rows of the vectors in shared
+// memory for the whole solve.  Entries hold the cluster address of the x
+// they multiply (its owner's copy), so a product is shared-memory loads, one
+// distributed-shared-memory gather and the multiply-adds, in the same order
+// as in the sliced-ELL kernels.  For a total, each warp's sum is pushed to
+// every CTA before the barrier and added there by one warp, which also does
+// the division; r.r travels with r.z.  Rows, threads and orders of the sums
+// are pcg_body's, so both give the same bits.  64 x 64 Laplacian, FSAI width 8 (GB300,
+// 16 CTAs): 13.4 us an iteration with pcg_body, 8.9 here.
+enum ResidentVec : int { V_P, V_R, V_Z, V_T, V_AP, V_X, V_U, V_IM, V_WM, V_COUNT };
+
+// Rows of a vector's part in each CTA; one more is zero for padding.
+__host__ __device__ constexpr size_t resident_vec_bytes(int smax) {
+  return ((size_t)smax * kSlice + 2) * sizeof(double);
+}
+__host__ __device__ constexpr size_t resident_bytes(int smax, const int (&wide)[3], int cluster) {
+  size_t b = resident_vec_bytes(smax) * V_COUNT;
+  b += 2 * 2 * sizeof(double) * (size_t)cluster * (kThreadsC / 32);  // two totals, two slots
+  for (int w : wide)
+    b += (size_t)smax * kSlice * w * (sizeof(double) + sizeof(uint32_t)) +
+         (size_t)smax * (kSlice * sizeof(uint32_t) + sizeof(int));
+  return (b + 15) & ~(size_t)15;
+}
+
+__device__ __forceinline__ uint32_t cluster_address(uint32_t own, int cta) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own), "r"(cta));
+  return a;
+}
+__device__ __forceinline__ double cluster_load(uint32_t a) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_store(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+constexpr uint32_t kNoRow = 0xffffffffu;
+
+struct ResidentMat {
+  double* vals;    // entry (j, k, lane) at (j * wide + k) * 32 + lane
+  uint32_t* addr;  // cluster address of x's V_P copy
+  uint32_t* out;   // [smax][32] cluster address of the row's V_P copy (kNoRow past the last)
+  int* width;      // [smax]
+  int wide;
+};
+
+__device__ void pcg_resident(const Args& a, int cta, int ncta, unsigned char* smem) {
+  cgr::cluster_group cl = cgr::this_cluster();
+  KrylovScalars* ks = a.ks;
+  const int n = (int)a.n, S = a.A.nslices, smax = a.smax;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kWarps = kThreadsC / 32;
+  const bool precond = a.G.nslices >= 0, factored = a.inv_mass != nullptr;
+  const int lo = cluster_slice(S, cta, ncta), own = cluster_slice(S, cta + 1, ncta) - lo;
+  const size_t vbytes = resident_vec_bytes(smax);
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(smem);
+  auto vec = [&](int v) { return reinterpret_cast<double*>(smem + v * vbytes); };
+  auto address = [&](int row) {
+    const int s = row / kSlice;
+    const int c = (int)((((int64_t)s + 1) * ncta - 1) / S);  // the CTA that owns s
+    const int first = cluster_slice(S, c, ncta) * kSlice;
+    return cluster_address(base + (uint32_t)(row - first) * 8u, c);
+  };
+  const uint32_t zero = cluster_address(base + (uint32_t)smax * kSlice * 8u, cta);
+  unsigned char* at = smem + vbytes * V_COUNT;
+  double* xch = reinterpret_cast<double*>(at);  // [slot][value][ncta * kWarps]
+  const int parts = ncta * kWarps;
+  at += 4 * sizeof(double) * parts;
+  ResidentMat M[3];
+  for (int q = 0; q < 3; ++q) {
+    M[q].wide = a.wide[q];
+    M[q].vals = reinterpret_cast<double*>(at);
+    at += sizeof(double) * (size_t)smax * kSlice * a.wide[q];
+  }
+  for (int q = 0; q < 3; ++q) {
+    M[q].addr = reinterpret_cast<uint32_t*>(at);
+    at += sizeof(uint32_t) * (size_t)smax * kSlice * a.wide[q];
+    M[q].out = reinterpret_cast<uint32_t*>(at);
+    at += sizeof(uint32_t) * (size_t)smax * kSlice;
+    M[q].width = reinterpret_cast<int*>(at);
+    at += sizeof(int) * (size_t)smax;
+  }
+  for (int q = 0; q < (precond ? 3 : 1); ++q) {
+    const Mat& m = q == 0 ? a.A : q == 1 ? a.G : a.GT;
+    for (int j = warp; j < own; j += kWarps) {
+      const int64_t first = m.slice_ptr[lo + j];
+      const int width = (int)((m.slice_ptr[lo + j + 1] - first) / kSlice);
+      if (lane == 0) M[q].width[j] = width;
+      const int row = (lo + j) * kSlice + lane;
+      M[q].out[j * kSlice + lane] = row < m.nrow ? address(m.perm ? m.perm[row] : row) : kNoRow;
+      for (int k = 0; k < width; ++k) {
+        const int64_t e = first + (int64_t)k * kSlice + lane;
+        const int c = m.cols[e];
+        const int to = (j * M[q].wide + k) * kSlice + lane;
+        M[q].vals[to] = m.vals[e];
+        M[q].addr[to] = c >= 0 ? address(c) : zero;
+      }
+    }
+  }
+  for (int i = threadIdx.x; i < smax * kSlice + 2; i += kThreadsC) {
+    const int row = lo * kSlice + i;
+    const bool in = i < own * kSlice && row < n;
+    for (int v = 0; v < V_COUNT; ++v) vec(v)[i] = 0.0;
+    if (in) {
+      vec(V_X)[i] = a.x[row];
+      if (factored) {
+        vec(V_IM)[i] = a.inv_mass[row];
+        vec(V_WM)[i] = a.wmass[row];
+      }
+    }
+  }
+  cl.sync();
+
+  // dst = m src (CoopEpi epilogues); returns this thread's share of dst . w.
+  auto product = [&](const ResidentMat& m, int src, int dst, int epi, int w, int mul) {
+    const uint32_t so = (uint32_t)(src * vbytes);
+    double dot = 0.0;
+    for (int j = warp; j < own; j += kWarps) {
+      const int width = m.width[j];
+      const double* v = m.vals + (size_t)j * m.wide * kSlice + lane;
+      const uint32_t* ad = m.addr + (size_t)j * m.wide * kSlice + lane;
+      double acc = 0.0;
+      for (int k0 = 0; k0 < width; k0 += 8) {
+        double xv[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          xv[k] = k0 + k < width ? cluster_load(ad[(k0 + k) * kSlice] + so) : 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k0 + k < width) acc = fma(v[(k0 + k) * kSlice], xv[k], acc);
+      }
+      const uint32_t row = m.out[j * kSlice + lane];
+      if (row != kNoRow) {
+        double out = acc;
+        if (epi == CE_SCALE) out = cluster_load(row + (uint32_t)(V_IM * vbytes)) * acc;
+        else if (epi == CE_MASS)
+          out = fma(cluster_load(row + (uint32_t)(V_WM * vbytes)),
+                    cluster_load(row + (uint32_t)(mul * vbytes)), acc);
+        cluster_store(row + (uint32_t)(dst * vbytes), out);
+        if (w >= 0) dot = fma(out, cluster_load(row + (uint32_t)(w * vbytes)), dot);
+      }
+    }
+    return dot;
+  };
+  auto apply_a = [&](int src, int dst, int w) {
+    if (!factored) return product(M[0], src, dst, CE_PLAIN, w, 0);
+    product(M[0], src, V_U, CE_SCALE, -1, 0);
+    cl.sync();
+    return product(M[0], V_U, dst, CE_MASS, w, src);
+  };
+  // Totals of two values over the cluster (pushed, one barrier, added in
+  // the order of the warps), and num / t0 or t1 / den; a barrier for
+  // everything stored before it.
+  __shared__ double sh[3];
+  int slot = 0;
+  double t0 = 0.0, t1 = 0.0, ratio = 0.0;
+  auto totals = [&](double v0, double v1, bool two, double num, double den) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+    if (two) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+    }
+    double* mine = xch + slot * 2 * parts;
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(mine + cta * kWarps + warp);
+    if (lane < ncta) {
+      cluster_store(cluster_address(to, lane), v0);
+      if (two) cluster_store(cluster_address(to + (uint32_t)parts * 8u, lane), v1);
+    }
+    cl.sync();
+    // Warp 0 adds the first value, warp 1 the second.
+    if (warp == 0 || (two && warp == 1)) {
+      double s = 0.0;
+      for (int q = lane; q < parts; q += 32) s += mine[warp * parts + q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) {
+        sh[warp] = s;
+        if (warp == (two ? 1 : 0)) sh[2] = two ? s / den : num / s;
+      }
+    }
+    __syncthreads();
+    t0 = sh[0];
+    t1 = sh[1];
+    ratio = sh[2];
+    __syncthreads();
+    slot ^= 1;
+  };
+
+  const double tol = ks->tol, atol = ks->atol;
+  const int maxiter = ks->maxiter;
+  double* hist = ks->hist;
+  const int hist_len = ks->hist_len;
+  const bool first_thread = cta == 0 && threadIdx.x == 0;
+  const int rows = min(own * kSlice, n - lo * kSlice);
+  double *x = vec(V_X), *r = vec(V_R), *z = vec(V_Z), *p = vec(V_P), *Ap = vec(V_AP);
+  apply_a(V_X, V_AP, -1);
+  cl.sync();
+  double pbb = 0.0, prr = 0.0;
+  for (int i = threadIdx.x; i < rows; i += kThreadsC) {
+    const double bi = a.b[lo * kSlice + i];
+    const double ri = bi - Ap[i];
+    r[i] = ri;
+    pbb = fma(bi, bi, pbb);
+    prr = fma(ri, ri, prr);
+  }
+  totals(pbb, prr, true, 1.0, 1.0);  // and r is visible to the cluster
+  const double bb = t0;
+  double rr = t1;
+  const double at_ = fmax(atol, tol * sqrt(bb));
+  const double atol_sq = at_ * at_;
+  if (first_thread && hist && hist_len > 0) hist[0] = sqrt(rr);
+  // z = M r; this thread's share of r.z.
+  auto precondition = [&]() {
+    if (precond) {
+      product(M[1], V_R, V_T, CE_PLAIN, -1, 0);
+      cl.sync();
+      return product(M[2], V_T, V_Z, CE_PLAIN, V_R, 0);
+    }
+    double d = 0.0;
+    for (int i = threadIdx.x; i < rows; i += kThreadsC) {
+      z[i] = r[i];
+      d = fma(r[i], r[i], d);
+    }
+    return d;
+  };
+  totals(0.0, precondition(), true, 1.0, 1.0);
+  double rz = t1;
+  for (int i = threadIdx.x; i < rows; i += kThreadsC) p[i] = z[i];
+  cl.sync();
+  int it = 0;
+  double alpha = 0.0, beta = 0.0, pap = 0.0;
+  while (rr > atol_sq && it < maxiter) {
+    totals(apply_a(V_P, V_AP, V_P), 0.0, false, rz, 1.0);
+    pap = t0;
+    alpha = ratio;
+    prr = 0.0;
+    for (int i = threadIdx.x; i < rows; i += kThreadsC) {
+      x[i] = fma(alpha, p[i], x[i]);
+      const double ri = fma(-alpha, Ap[i], r[i]);
+      r[i] = ri;
+      prr = fma(ri, ri, prr);
+    }
+    cl.sync();
+    totals(prr, precondition(), true, 1.0, rz);
+    rr = t0;
+    beta = ratio;
+    rz = t1;
+    if (first_thread && hist && it + 1 < hist_len) hist[it + 1] = sqrt(rr);
+    ++it;
+    for (int i = threadIdx.x; i < rows; i += kThreadsC) p[i] = fma(beta, p[i], z[i]);
+    cl.sync();
+  }
+  for (int i = threadIdx.x; i < rows; i += kThreadsC) a.x[lo * kSlice + i] = x[i];
+  // No CTA leaves while another may still use its shared memory.
+  cl.sync();
+  if (first_thread) {
     ks->bb = bb;
     ks->atol_sq = atol_sq;
     ks->rr = rr;
@@ -423,10 +706,15 @@ __device__ void pcg_body(const Args& a, S& grid, int cta, int ncta, double* sh) 
 
 // One system on one cluster (the grid is that cluster).
 __global__ void __launch_bounds__(kThreadsC) pcg_kernel(Args a) {
-  __shared__ double sh[kThreadsC / 32 + 1];
-  __shared__ double xch[2];
+  extern __shared__ __align__(16) unsigned char coop_smem[];
+  if (a.smax > 0) {
+    pcg_resident(a, blockIdx.x, gridDim.x, coop_smem);
+    return;
+  }
+  __shared__ double sh;
+  __shared__ double xch[2 * kThreadsC / 32];
   ClusterSync grid(xch);
-  pcg_body(a, grid, blockIdx.x, gridDim.x, sh);
+  pcg_body(a, grid, blockIdx.x, gridDim.x, &sh);
 }
 
 // Many systems in one launch: cluster c (CTAs c*C .. c*C+C-1 of a 1-D grid
@@ -434,15 +722,20 @@ __global__ void __launch_bounds__(kThreadsC) pcg_kernel(Args a) {
 // preconditioner, vectors and scalars.  Clusters never wait on each other:
 // each leaves when its own system has converged.
 __global__ void __launch_bounds__(kThreadsC) multi_cluster_kernel(const Args* systems, int nsys) {
-  __shared__ double sh[kThreadsC / 32 + 1];
-  __shared__ double xch[2];
+  __shared__ double sh;
+  __shared__ double xch[2 * kThreadsC / 32];
   cgr::cluster_group cl = cgr::this_cluster();
   const int C = (int)cl.num_blocks();
   const int sys = blockIdx.x / C;
   if (sys >= nsys) return;  // uniform over a cluster
   const Args a = systems[sys];
+  extern __shared__ __align__(16) unsigned char coop_smem[];
+  if (a.smax > 0) {
+    pcg_resident(a, (int)cl.block_rank(), C, coop_smem);
+    return;
+  }
   ClusterSync sync(xch);
-  pcg_body(a, sync, (int)cl.block_rank(), C, sh);
+  pcg_body(a, sync, (int)cl.block_rank(), C, &sh);
 }
 
 // tol, atol, maxiter (<= 0: the system's size) of every system, no history.
@@ -523,6 +816,60 @@ int cluster_size() {
   return chosen;
 }
 
+// Shared memory per CTA a resident system may take (0: no resident path),
+// schedulable with both kernels at the cluster size they run with.
+size_t resident_limit() {
+  static const size_t limit = [] {
+    const int c = cluster_size();
+    const void* kerns[2] = {(const void*)pcg_kernel, (const void*)multi_cluster_kernel};
+    for (size_t bytes : {(size_t)208 << 10, (size_t)100 << 10}) {
+      bool ok = c > 0;
+      for (const void* k : kerns) {
+        if (!ok) break;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+            cudaSuccess) {
+          cudaGetLastError();
+          ok = false;
+          break;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(c);
+        cfg.blockDim = dim3(kThreadsC);
+        cfg.dynamicSmemBytes = bytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = c;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+          cudaGetLastError();
+          ok = false;
+        }
+      }
+      if (ok) return bytes;
+    }
+    return (size_t)0;
+  }();
+  return limit;
+}
+
+// Makes a system resident when it fits `limit` bytes a CTA.  Returns its
+// shared memory.
+size_t choose_resident(Args& a, const Sell* A, const Sell* G, const Sell* GT, int cluster,
+                       size_t limit) {
+  a.smax = 0;
+  const int smax = (A->nslices + cluster - 1) / cluster;
+  const int wide[3] = {A->widest, G ? G->widest : 0, GT ? GT->widest : 0};
+  const size_t bytes = resident_bytes(smax, wide, cluster);
+  if (smax < 1 || bytes > limit) return 0;
+  a.smax = smax;
+  for (int q = 0; q < 3; ++q) a.wide[q] = wide[q];
+  return bytes;
+}
+
 }  // namespace coop
 
 struct Solver {
@@ -545,6 +892,7 @@ struct Solver {
   // and an FSAI or no preconditioner run as one kernel on one cluster.
   bool coop = false;
   int coop_cluster = 0;  // CTAs of that cluster
+  size_t coop_smem = 0;  // their shared memory (systems that fit it)
   coop::Args cargs{};
   DevBuf store;  // of r .. ks
   DevBuf r, z, p, Ap, Az, y, ks, zeros, t, u;
@@ -808,6 +1156,8 @@ struct Solver {
     cargs.Ap = Ap.as<double>();
     cargs.t = t.as<double>();
     cargs.ks = K();
+    coop_smem = coop::choose_resident(cargs, pa[0], M ? pm[0] : nullptr, M ? pm[1] : nullptr,
+                                      coop_cluster, coop::resident_limit());
     coop = true;
     return GBPC_OK;
   }
@@ -825,6 +1175,7 @@ struct Solver {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(coop_cluster);
       cfg.blockDim = dim3(coop::kThreadsC);
+      cfg.dynamicSmemBytes = coop_smem;
       cfg.stream = st;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1040,6 +1391,7 @@ struct gbpc_csolver {
   size_t device_bytes = 0;  // declared first: released last
   int nsys = 0;
   int cluster = 0;
+  size_t smem = 0;  // per CTA, the most that one of the systems takes
   std::vector<coop::Args> host_args;
   gbpc::DevBuf args, vecs, scalars;
 };
@@ -1111,6 +1463,12 @@ extern "C" int gbpc_csolver_create(int nsys, gbpc_op* const* A, gbpc_op* const* 
     return rc;
   }
   h->host_args.resize((size_t)nsys);
+  // More clusters than the GPU holds at one CTA an SM: keep two on each
+  // (32 tet cubes of 17-20 vertices a side, GB300: 45 ms from L2 with several
+  // CTAs an SM, 65 ms from shared memory with one).
+  const size_t limit = (int64_t)nsys * C <= kSms
+                           ? coop::resident_limit()
+                           : std::min(coop::resident_limit(), (size_t)100 << 10);
   double* v = h->vecs.as<double>();
   for (int s = 0; s < nsys; ++s) {
     const Parts& p = parts[s];
@@ -1135,6 +1493,7 @@ extern "C" int gbpc_csolver_create(int nsys, gbpc_op* const* A, gbpc_op* const* 
     g.u = p.im ? v + 5 * p.n : nullptr;
     v += (size_t)p.n * (p.im ? 6 : 5);
     g.ks = h->scalars.as<KrylovScalars>() + s;
+    h->smem = std::max(h->smem, coop::choose_resident(g, p.a, p.g, p.gt, C, limit));
   }
   *out = h;
   return GBPC_OK;
@@ -1167,6 +1526,7 @@ extern "C" int gbpc_csolver_run(gbpc_csolver* h, int count, const double* const*
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)count * h->cluster);
   cfg.blockDim = dim3(coop::kThreadsC);
+  cfg.dynamicSmemBytes = h->smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

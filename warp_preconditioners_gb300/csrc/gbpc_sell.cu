@@ -525,6 +525,7 @@ int sell_build(Sell& s, int nrow_out, int ncol, int B, const int32_t* off, const
     GBPC_CUDA_TRY(cudaStreamSynchronize(st));
   }
   s.nent = h.nent;
+  s.widest = h.widest;
   if ((rc = alloc_group(s.store, {{&s.slice_ptr, sizeof(int64_t) * (ns + 1)},
                                   {&s.sched, sizeof(int4) * ns},
                                   {&s.err, sizeof(int32_t)},
