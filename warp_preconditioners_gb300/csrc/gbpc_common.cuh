@@ -119,8 +119,8 @@ struct KrylovScalars {
   double bb;       // b.b
   double atol_sq;  // max(atol, tol |b|)^2
   double rr;       // recursive r.r
-  double rz;       // CG: r.z   | CR: z.Az
-  double rz_new;
+  double rz;       // CG: r.z of the step being taken | CR: z.Az
+  double rz_new;   // CG: the newest r.z
   double denom;    // CG: p.Ap  | CR: y.Ap
   double alpha;
   double beta;
@@ -133,7 +133,7 @@ struct KrylovScalars {
   double atol;
   double* hist;    // residual history: hist[k] = |r_k| for k < hist_len (nullptr: none)
   int hist_len;
-  int pad2;
+  unsigned parts;  // CG: CTAs that wrote the partial sums of the last product
 };
 
 // What the last CTA does with a finished reduction.
@@ -142,11 +142,14 @@ enum FinMode : int {
   FIN_STORE = 1,       // *out = total
   FIN_INIT_BB = 2,     // bb = total
   FIN_INIT_RR = 3,     // rr = total; atol_sq; active; graph condition
-  FIN_CG_ALPHA = 4,    // denom = total; alpha = rz / denom
-  FIN_RR = 5,          // rr = total
-  FIN_CG_BETA = 6,     // beta = total / rz; rz = total; it++; active
-  FIN_INIT_RZ = 7,     // rz = total
-  FIN_CR_ALPHA = 8,    // denom = total; alpha = rz / denom  (rz holds z.Az)
+  FIN_RR = 4,          // rr = total
+  FIN_CR_BETA = 5,     // beta = total / rz; rz = total; it++; active
+  FIN_INIT_RZ = 6,     // rz = rz_new = total
+  FIN_CR_ALPHA = 7,    // denom = total; alpha = rz / denom  (rz holds z.Az)
+  // The CTAs leave their partial sums and nothing else; the next kernel of
+  // the CG loop adds them (warp_total).
+  FIN_DEFER = 8,        // parts = the number of CTAs
+  FIN_DEFER_UPDATE = 9, // of the vector update: its consumer has the same grid
 };
 
 struct Reduction {
@@ -232,8 +235,8 @@ __device__ __forceinline__ void finalize(const Reduction& red, double total) {
     }
     case FIN_INIT_RZ:
       ks->rz = total;
+      ks->rz_new = total;
       break;
-    case FIN_CG_ALPHA:
     case FIN_CR_ALPHA:
       ks->denom = total;
       ks->alpha = ks->rz / total;
@@ -243,8 +246,7 @@ __device__ __forceinline__ void finalize(const Reduction& red, double total) {
       // The iteration count is advanced later in the same iteration.
       if (ks->hist && ks->it + 1 < ks->hist_len) ks->hist[ks->it + 1] = sqrt(total);
       break;
-    case FIN_CG_BETA:
-      ks->rz_new = total;
+    case FIN_CR_BETA:
       ks->beta = total / ks->rz;
       ks->rz = total;
       ks->it += 1;
@@ -255,17 +257,55 @@ __device__ __forceinline__ void finalize(const Reduction& red, double total) {
   }
 }
 
-// Every thread of the CTA calls this with its partial; the last CTA to arrive
-// sums all CTA partials and applies the finalize action.  That final sum is
-// one warp's: lane l adds partials l, l + 32, ... (loads issued kFinLoads at
-// a time), then a fixed butterfly — fewer barriers and dependent FP64 adds
-// on the critical path than a whole-CTA sum, and the same order every run.
+// Sum of the partials of `count` CTAs by one full warp, in every lane: lane l
+// adds partials l, l + 32, ... (loads issued L at a time), then a fixed
+// butterfly — fewer barriers and dependent FP64 adds on the critical path
+// than a whole-CTA sum, and the same order every run.  The buffer holds at
+// least 32 * L doubles whatever the count, so the first loads wait for
+// nothing; what lies past the count is not added.
 constexpr int kFinLoads = 10;  // 320 partials per pass: every grid of kSms * kCtasPerSm CTAs
+constexpr int kUpdatePartials = 608;  // where the vector update's partials begin (FIN_DEFER_UPDATE)
 
+template <int L = kFinLoads, typename Count>
+__device__ __forceinline__ double warp_total(const double* partials, Count&& count_of) {
+  const unsigned lane = threadIdx.x & 31;
+  double p[L];
+#pragma unroll
+  for (int q = 0; q < L; ++q) p[q] = __ldcg(partials + lane + 32 * q);
+  const unsigned count = count_of();
+  double acc = 0.0;
+  for (unsigned b = 0;;) {
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      if (b + 32 * q >= count) break;  // an add costs its issue slots whatever it adds
+      acc += b + lane + 32 * q < count ? p[q] : 0.0;
+    }
+    b += 32 * L;
+    if (b >= count) break;
+#pragma unroll
+    for (int q = 0; q < L; ++q)
+      p[q] = b + lane + 32 * q < count ? __ldcg(partials + b + lane + 32 * q) : 0.0;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  return acc;
+}
+
+// Every thread of the CTA calls this with its partial; the last CTA to arrive
+// sums all CTA partials and applies the finalize action (the FIN_DEFER modes
+// leave the sum to the next kernel: no fence, no arrival counter, no CTA that
+// works on alone while the others' SMs are idle).
 __device__ __forceinline__ void reduce_and_finalize(const Reduction& red, double v) {
   __shared__ double smem[kThreads];
   __shared__ bool am_last;
   const double s = block_sum(v, smem);
+  if (red.mode >= FIN_DEFER) {
+    if (threadIdx.x == 0) {
+      red.partials[blockIdx.x] = s;
+      if (red.mode == FIN_DEFER && blockIdx.x == 0) red.ks->parts = gridDim.x;
+    }
+    return;
+  }
   if (threadIdx.x == 0) {
     red.partials[blockIdx.x] = s;
     __threadfence();
@@ -275,21 +315,8 @@ __device__ __forceinline__ void reduce_and_finalize(const Reduction& red, double
   __syncthreads();
   if (am_last && threadIdx.x < 32) {
     __threadfence();
-    const unsigned lane = threadIdx.x, count = gridDim.x;
-    double acc = 0.0;
-    for (unsigned b = 0; b < count; b += 32 * kFinLoads) {
-      double p[kFinLoads];
-#pragma unroll
-      for (int q = 0; q < kFinLoads; ++q) {
-        const unsigned k = b + lane + 32 * q;
-        p[q] = k < count ? __ldcg(red.partials + k) : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q < kFinLoads; ++q) acc += p[q];
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (lane == 0) {
+    const double acc = warp_total(red.partials, [] { return gridDim.x; });
+    if (threadIdx.x == 0) {
       *red.counter = 0u;
       finalize(red, acc);
     }

@@ -39,12 +39,24 @@ __device__ __forceinline__ bool inactive(const KrylovScalars* ks) {
   return *(volatile const int*)&ks->active == 0;
 }
 
-// x += alpha p; r -= alpha Ap; reduce r.r.  R32: also r32 = (float) r, the
-// input of a float32-applied preconditioner (no separate conversion pass).
+constexpr int kProductLoads = 5;  // 160 partials: every grid of kSms CTAs
+
+// alpha = r.z / p.Ap; x += alpha p; r -= alpha Ap; reduce r.r.  R32: also
+// r32 = (float) r, the input of a float32-applied preconditioner (no separate
+// conversion pass).
+//
+// p.Ap arrives as the product's partial sums (`pAp`): one warp of each CTA
+// adds them while the CTA's rows are loaded.  The last CTA of the product
+// doing it costs a fence, an arrival counter and a division with the rest of
+// the chip idle: an iteration (this kernel, cg_direction_kernel and four
+// products) on the squared Laplacian of a 70^3 tetrahedral cube took 78.8 us
+// with the sums there and takes 74.7 us with them here.  The sums have the
+// same terms in the same order either way.
 template <bool R32>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 cg_update_kernel(int64_t n, KrylovScalars* ks, double* x, double* r, const double* p,
-                 const double* Ap, float* r32, Reduction red) {
+                 const double* Ap, float* r32, const double* pAp, Reduction red) {
+  __shared__ double step;
   // x and p are not written by the previous kernel (the operator apply that
   // produced Ap), so a thread's first row of them is read before the wait.
   const int64_t i0 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -55,13 +67,32 @@ cg_update_kernel(int64_t n, KrylovScalars* ks, double* x, double* r, const doubl
   }
   pdl_wait();
   pdl_launch_dependents();
+  double r0 = 0.0, w0 = 0.0;
+  if (i0 < n) {
+    r0 = r[i0];
+    w0 = Ap[i0];
+  }
   if (inactive(ks)) return;
-  const double alpha = ks->alpha;
+  if (threadIdx.x < 32) {
+    const double rz = ks->rz_new;
+    const double denom = warp_total<kProductLoads>(pAp, [&] { return *(volatile unsigned*)&ks->parts; });
+    if (threadIdx.x == 0) {
+      const double a = rz / denom;
+      step = a;
+      if (blockIdx.x == 0) {
+        ks->denom = denom;
+        ks->alpha = a;
+        ks->rz = rz;  // no CTA of this kernel reads it
+      }
+    }
+  }
+  __syncthreads();
+  const double alpha = step;
   double part = 0.0;
   for (int64_t i = i0; i < n; i += (int64_t)gridDim.x * kThreads) {
     const bool first = i == i0;
     x[i] = fma(alpha, first ? p0 : p[i], first ? x0 : x[i]);
-    const double ri = fma(-alpha, Ap[i], r[i]);
+    const double ri = fma(-alpha, first ? w0 : Ap[i], first ? r0 : r[i]);
     r[i] = ri;
     if (R32) r32[i] = (float)ri;
     part = fma(ri, ri, part);
@@ -89,20 +120,64 @@ cr_update_kernel(int64_t n, KrylovScalars* ks, double* x, double* r, double* z, 
   reduce_and_finalize(red, part);
 }
 
-// p = z + beta p  (and q = w + beta q with Q: CR).  Q is a template
-// parameter so that CG issues no FP64 instruction for the absent q.  Z is
-// float for a float32-applied preconditioner (z widened on the fly).
-template <bool Q, typename Z = double>
+// CG: beta = new r.z / r.z; p = z + beta p; end of the iteration.  r.z
+// arrives as the preconditioner's partial sums (`rzp`), r.r as the vector
+// update's (`rrp`, of as many CTAs as this grid has).  CTA 0 keeps the
+// scalars: no other CTA reads what it writes, but for `active`, which turns 0
+// only after the last iteration, whose p nothing uses.  Z is float for a
+// float32-applied preconditioner (z widened on the fly).
+template <typename Z>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
-xpay_kernel(int64_t n, const KrylovScalars* ks, const Z* z, double* p, const double* w,
-            double* q) {
-  // p (and q) were last written an iteration ago, not by the previous
-  // kernel: a thread's first row of them is read before the wait.
+cg_direction_kernel(int64_t n, KrylovScalars* ks, const Z* z, double* p, const double* rzp,
+                    const double* rrp) {
+  __shared__ double sums[2], step;
+  // p was last written an iteration ago, not by the previous kernel: a
+  // thread's first row of it is read before the wait.
+  const int64_t i0 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+  const double p0 = i0 < n ? p[i0] : 0.0;
+  pdl_wait();
+  pdl_launch_dependents();
+  const double z0 = i0 < n ? (double)z[i0] : 0.0;
+  if (inactive(ks)) return;
+  if (threadIdx.x < 32) {
+    const double rz = ks->rz;
+    const double t = warp_total<kProductLoads>(rzp, [&] { return *(volatile unsigned*)&ks->parts; });
+    if (threadIdx.x == 0) {
+      sums[0] = t;
+      step = t / rz;
+    }
+  } else if (threadIdx.x < 64 && blockIdx.x == 0) {
+    const double t = warp_total(rrp, [] { return gridDim.x; });
+    if (threadIdx.x == 32) sums[1] = t;
+  }
+  __syncthreads();
+  const double beta = step;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int it = ks->it;
+    ks->rz_new = sums[0];
+    ks->beta = beta;
+    ks->rr = sums[1];
+    if (ks->hist && it + 1 < ks->hist_len) ks->hist[it + 1] = sqrt(sums[1]);
+    ks->it = it + 1;
+    set_active(ks);
+  }
+  for (int64_t i = i0; i < n; i += (int64_t)gridDim.x * kThreads) {
+    const bool first = i == i0;
+    p[i] = fma(beta, first ? p0 : p[i], first ? z0 : (double)z[i]);
+  }
+}
+
+// CR: p = z + beta p; q = w + beta q.
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
+cr_direction_kernel(int64_t n, const KrylovScalars* ks, const double* z, double* p,
+                    const double* w, double* q) {
+  // p and q were last written an iteration ago, not by the previous kernel:
+  // a thread's first row of them is read before the wait.
   const int64_t i0 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
   double p0 = 0.0, q0 = 0.0;
   if (i0 < n) {
     p0 = p[i0];
-    if (Q) q0 = q[i0];
+    q0 = q[i0];
   }
   pdl_wait();
   pdl_launch_dependents();
@@ -110,8 +185,8 @@ xpay_kernel(int64_t n, const KrylovScalars* ks, const Z* z, double* p, const dou
   const double beta = ks->beta;
   for (int64_t i = i0; i < n; i += (int64_t)gridDim.x * kThreads) {
     const bool first = i == i0;
-    p[i] = fma(beta, first ? p0 : p[i], (double)z[i]);
-    if (Q) q[i] = fma(beta, first ? q0 : q[i], w[i]);
+    p[i] = fma(beta, first ? p0 : p[i], z[i]);
+    q[i] = fma(beta, first ? q0 : q[i], w[i]);
   }
 }
 
@@ -158,6 +233,9 @@ __global__ void copy_outputs_kernel(const KrylovScalars* ks, int32_t* nit, doubl
   if (atol_sq) *atol_sq = ks->atol_sq;
 }
 
+static_assert(kSms * kCtasPerSm <= kUpdatePartials &&
+                  kUpdatePartials + kSms * kCtasPerSm <= kMaxCtas && 32 * kFinLoads <= kUpdatePartials,
+              "a CG iteration's two sets of partial sums share one reduction buffer");
 int vec_grid(int64_t n) { return std::min<int64_t>(grid_for(n, kThreads), kSms * kCtasPerSm); }
 
 }  // namespace
@@ -988,38 +1066,43 @@ struct Solver {
     rrr.mode = FIN_RR;
     rrr.ks = K();
     rrr.w = r.as<double>();
+    const double* parts = rb.partials.as<double>();
+    if (method == GBPC_CG) {
+      rrr.partials += kUpdatePartials;
+      rrr.mode = FIN_DEFER_UPDATE;
+    }
     if (method == GBPC_CG && low) {
-      DotSpec da = dot(p.as<double>(), FIN_CG_ALPHA);
+      DotSpec da = dot(p.as<double>(), FIN_DEFER);
       if ((rc = A->apply(p.p, nullptr, Ap.p, 1.0, 0.0, guard, &da, st))) return rc;
       GBPC_CUDA_TRY(launch_k(cg_update_kernel<true>, vec_grid(n), kThreads, 0, st, n, K(), x,
                              r.as<double>(), (const double*)p.as<double>(),
-                             (const double*)Ap.as<double>(), low->in32.as<float>(), rrr));
-      DotSpec db = dot(r.as<double>(), FIN_CG_BETA);
+                             (const double*)Ap.as<double>(), low->in32.as<float>(), parts, rrr));
+      DotSpec db = dot(r.as<double>(), FIN_DEFER);
       if ((rc = low->inner->apply(low->in32.p, nullptr, low->out32.p, 1.0, 0.0, guard, &db, st)))
         return rc;
-      GBPC_CUDA_TRY(launch_k(xpay_kernel<false, float>, vec_grid(n), kThreads, 0, st, n,
-                             (const KrylovScalars*)K(), (const float*)low->out32.as<float>(),
-                             p.as<double>(), (const double*)nullptr, (double*)nullptr));
+      GBPC_CUDA_TRY(launch_k(cg_direction_kernel<float>, vec_grid(n), kThreads, 0, st, n, K(),
+                             (const float*)low->out32.as<float>(), p.as<double>(), parts,
+                             parts + kUpdatePartials));
     } else if (method == GBPC_CG) {
-      DotSpec da = dot(p.as<double>(), FIN_CG_ALPHA);
+      DotSpec da = dot(p.as<double>(), FIN_DEFER);
       if ((rc = A->apply(p.p, nullptr, Ap.p, 1.0, 0.0, guard, &da, st))) return rc;
       GBPC_CUDA_TRY(launch_k(cg_update_kernel<false>, vec_grid(n), kThreads, 0, st, n, K(), x,
                              r.as<double>(), (const double*)p.as<double>(),
-                             (const double*)Ap.as<double>(), (float*)nullptr, rrr));
-      DotSpec db = dot(r.as<double>(), FIN_CG_BETA);
+                             (const double*)Ap.as<double>(), (float*)nullptr, parts, rrr));
+      DotSpec db = dot(r.as<double>(), FIN_DEFER);
       if ((rc = precondition(r.as<double>(), z.as<double>(), guard, &db, st))) return rc;
-      GBPC_CUDA_TRY(launch_k(xpay_kernel<false>, vec_grid(n), kThreads, 0, st, n,
-                             (const KrylovScalars*)K(), (const double*)z.as<double>(),
-                             p.as<double>(), (const double*)nullptr, (double*)nullptr));
+      GBPC_CUDA_TRY(launch_k(cg_direction_kernel<double>, vec_grid(n), kThreads, 0, st, n, K(),
+                             (const double*)z.as<double>(), p.as<double>(), parts,
+                             parts + kUpdatePartials));
     } else {
       DotSpec da = dot(Ap.as<double>(), FIN_CR_ALPHA);
       if ((rc = precondition(Ap.as<double>(), y.as<double>(), guard, &da, st))) return rc;
       GBPC_CUDA_TRY(launch_k(cr_update_kernel, vec_grid(n), kThreads, 0, st, n, K(), x,
                              r.as<double>(), z.as<double>(), (const double*)p.as<double>(),
                              (const double*)Ap.as<double>(), (const double*)y.as<double>(), rrr));
-      DotSpec db = dot(z.as<double>(), FIN_CG_BETA);
+      DotSpec db = dot(z.as<double>(), FIN_CR_BETA);
       if ((rc = A->apply(z.p, nullptr, Az.p, 1.0, 0.0, guard, &db, st))) return rc;
-      GBPC_CUDA_TRY(launch_k(xpay_kernel<true>, vec_grid(n), kThreads, 0, st, n,
+      GBPC_CUDA_TRY(launch_k(cr_direction_kernel, vec_grid(n), kThreads, 0, st, n,
                              (const KrylovScalars*)K(), (const double*)z.as<double>(),
                              p.as<double>(), (const double*)Az.as<double>(), Ap.as<double>()));
     }
