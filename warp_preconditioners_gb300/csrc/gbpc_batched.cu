@@ -13,7 +13,7 @@
 //
 // Dots are accumulated in float64 per right-hand side, folded across the row
 // groups of a warp, reduced per CTA through shared memory and combined in
-// index order by the last CTA to finish (deterministic for a given k).  Every
+// index order by the last to finish (deterministic for a given k).  Every
 // right-hand side has its own CG scalars and stopping test; finished ones are
 // masked out while the rest continue.
 
@@ -34,6 +34,9 @@ constexpr int kB = 32;            // lanes = right-hand sides per warp
 constexpr int kBThreads = 512;    // 16 warps per CTA
 constexpr int kBWarps = kBThreads / 32;
 constexpr int kBMaxCtas = 152 * 4;
+constexpr int kBUpdateRows = 4;          // rows that a warp of the update has in flight
+constexpr int kBResidentCtas = 152 * 2;  // CTAs of the products and the update: all resident
+static_assert(kBMaxCtas <= 2 * kBResidentCtas, "a product's CTA takes one or two shares of rows");
 
 struct BatchScalars {
   double bb[kB], atol_sq[kB], rr[kB], rz[kB], denom[kB], alpha[kB], beta[kB];
@@ -56,8 +59,8 @@ enum BFin : int {
 
 struct BRed {
   const void* w;     // dot(w, out) per right-hand side (nullptr: none); same type as out
-  double* partials;  // [gridDim.x][kB]
-  unsigned int* counter;
+  double* partials;  // [kBMaxCtas][kB], then the group sums [kBGroups][kB]
+  unsigned int* counter;  // [1 + kBGroups], zero between uses
   int mode;
   BatchScalars* bs;
   double* out;
@@ -100,8 +103,10 @@ __device__ __forceinline__ void b_set_active(BatchScalars* bs, int j, bool valid
   bs->active[j] = a;
 }
 
-// Per-RHS finalize, executed by lane j of warp 0 of the last CTA.
-__device__ __forceinline__ void b_finalize(const BRed& red, int j, double total) {
+// Per-RHS finalize, executed by lane j of the warp that has the total; rz and
+// active are the right-hand side's, read while the partial sums were.
+__device__ __forceinline__ void b_finalize(const BRed& red, int j, double total, double rz,
+                                           int active) {
   BatchScalars* bs = red.bs;
   const bool valid = j < bs->k;
   switch (red.mode) {
@@ -117,12 +122,12 @@ __device__ __forceinline__ void b_finalize(const BRed& red, int j, double total)
     case BF_INIT_RZ: bs->rz[j] = total; break;
     case BF_ALPHA:
       bs->denom[j] = total;
-      bs->alpha[j] = bs->active[j] ? bs->rz[j] / total : 0.0;
+      bs->alpha[j] = active ? rz / total : 0.0;
       break;
     case BF_RR: bs->rr[j] = total; break;
     case BF_BETA:
-      if (bs->active[j]) {
-        bs->beta[j] = total / bs->rz[j];
+      if (active) {
+        bs->beta[j] = total / rz;
         bs->rz[j] = total;
         bs->it[j] += 1;
       } else {
@@ -144,56 +149,95 @@ __device__ __forceinline__ void b_finalize(const BRed& red, int j, double total)
   }
 }
 
-// Every thread calls this with its lane's partial (lane = RHS).  Warps are
-// reduced through shared memory, CTAs through `partials` in index order.
-__device__ __forceinline__ void b_reduce(const BRed& red, double v) {
-  __shared__ double sm[kBWarps][kB];
-  __shared__ bool am_last;
+// One warp hands in partial sum `part` of `parts` (lane = RHS).  Group w of
+// them (w, w + kBGroups, ...) is added by the warp that hands in its last,
+// and the group sums, in order, by the group that is complete last.  An FP64
+// add of one warp costs its SM partition as much as any other: all of 608
+// partial sums added by one CTA (152 adds to a partition) took 5 us in which
+// every other SM was idle; spread over 16 warps of different CTAs it takes a
+// chain of 38 adds on each.
+constexpr int kBGroups = 16;
+
+__device__ __forceinline__ void b_hand_in(const BRed& red, double s, unsigned part,
+                                          unsigned parts) {
+  const int lane = threadIdx.x & 31;
+  red.partials[(size_t)part * kB + lane] = s;
+  __threadfence();
+  __syncwarp();
+  const unsigned group = part % kBGroups;
+  unsigned t = 0;
+  if (lane == 0) t = atomicAdd(red.counter + 1 + group, 1u);
+  if (__shfl_sync(0xffffffffu, t, 0) != (parts - group + kBGroups - 1) / kBGroups - 1) return;
+  __threadfence();
+  // Eight partials are loaded while the eight before them are added.
+  constexpr int G = 8;
+  s = 0.0;
+  double p[G];
+  auto load = [&](unsigned c, double (&d)[G]) {
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      const unsigned k = c + q * kBGroups;
+      d[q] = k < parts ? __ldcg(red.partials + (size_t)k * kB + lane) : 0.0;
+    }
+  };
+  load(group, p);
+  for (unsigned c = group; c < parts; c += G * kBGroups) {
+    double next[G];
+    load(c + G * kBGroups, next);
+#pragma unroll
+    for (int q = 0; q < G; ++q) {
+      if (c + q * kBGroups >= parts) break;
+      s += p[q];
+      p[q] = next[q];
+    }
+  }
+  double* sums = red.partials + (size_t)kBMaxCtas * kB;
+  sums[(size_t)group * kB + lane] = s;
+  __threadfence();
+  __syncwarp();
+  const unsigned groups = parts < kBGroups ? parts : kBGroups;
+  if (lane == 0) {
+    red.counter[1 + group] = 0u;
+    t = atomicAdd(red.counter, 1u);
+  }
+  if (__shfl_sync(0xffffffffu, t, 0) != groups - 1) return;
+  __threadfence();
+  double rz = 0.0;
+  int active = 0;
+  if (red.bs) {
+    rz = red.bs->rz[lane];
+    active = red.bs->active[lane];
+  }
+  double g[kBGroups];
+#pragma unroll
+  for (int q = 0; q < kBGroups; ++q) g[q] = q < groups ? __ldcg(sums + (size_t)q * kB + lane) : 0.0;
+  double total = g[0];
+#pragma unroll
+  for (int q = 1; q < kBGroups; ++q) {
+    if (q >= groups) break;
+    total += g[q];
+  }
+  b_finalize(red, lane, total, rz, active);
+  if (lane == 0) *red.counter = 0u;
+}
+
+// Every thread calls this with its lane's sums: of partial sum blockIdx.x
+// and, with n == 2, of partial sum blockIdx.x + gridDim.x.  Warps are reduced
+// through shared memory in index order.  Nothing follows in the calling
+// kernels, so the other warps leave at once.
+template <int N>
+__device__ __forceinline__ void b_reduce(const BRed& red, const double (&v)[N], int n,
+                                         unsigned parts) {
+  __shared__ double sm[N][kBWarps][kB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  sm[warp][lane] = v;
+#pragma unroll
+  for (int h = 0; h < N; ++h) sm[h][warp][lane] = v[h];
   __syncthreads();
-  if (warp == 0) {
-    double s = sm[0][lane];
+  if (warp >= n) return;
+  double s = sm[warp][0][lane];
 #pragma unroll
-    for (int w = 1; w < kBWarps; ++w) s += sm[w][lane];
-    red.partials[(size_t)blockIdx.x * kB + lane] = s;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const unsigned int t = atomicAdd(red.counter, 1u);
-    am_last = (t == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (am_last) {
-    // All warps of the last CTA sum a fixed subset of the CTA partials, then
-    // warp 0 adds the warp sums in order: deterministic and short.
-    __threadfence();
-    double s = 0.0;
-    unsigned int c = warp;
-    // Eight CTA partials loaded together (zero past the last CTA), added in
-    // the same order as one at a time: the loads no longer wait on each
-    // other, including the last, partial group.
-    for (; c < gridDim.x; c += 8 * kBWarps) {
-      double v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const unsigned int k = c + q * kBWarps;
-        v[q] = k < gridDim.x ? __ldcg(red.partials + (size_t)k * kB + lane) : 0.0;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) s += v[q];
-    }
-    sm[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0) {
-      double t = sm[0][lane];
-#pragma unroll
-      for (int w = 1; w < kBWarps; ++w) t += sm[w][lane];
-      b_finalize(red, lane, t);
-      if (lane == 0) *red.counter = 0u;
-    }
-  }
+  for (int w = 1; w < kBWarps; ++w) s += sm[warp][w][lane];
+  b_hand_in(red, s, blockIdx.x + warp * gridDim.x, parts);
 }
 
 enum BEpi : int { BE_AXPBY = 0, BE_SQLAP_BWD = 1 };
@@ -204,36 +248,103 @@ enum BEpi : int { BE_AXPBY = 0, BE_SQLAP_BWD = 1 };
 // scaled matrix.  Each row sums its entries in storage order, whatever KP.
 // UNIT: alpha == 1 and beta == 0 known at compile time (the Krylov loops'
 // products), so no scaling or Y term is issued.
+//
+// FP64 issue bounds it (28 us for the 14 entries a row of a 33^3 tetrahedral
+// Laplacian with 32 right-hand sides), so the rest is to keep every partition
+// issuing from start to end: two CTAs an SM, all resident, each taking two of
+// the `parts` shares of the rows (one share a CTA in two waves: 38.6 us, the
+// second wave starts cold while the first drains), a row's entries read one
+// row ahead of their use.  35.7 us now; with a dot product 48.6 -> 44.5 us.
 template <typename V, typename T, int EPI, bool DOT, int KP, bool UNIT = false>
 __global__ void __launch_bounds__(kBThreads, 2)
 bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __restrict__ col,
              const V* __restrict__ val, const T* X, const T* Y, T* Z, double alpha, double beta,
              int alpha_zero, int alpha_one, int beta_zero, const T* wm, const T* X2,
-             const int* guard, BRed red) {
+             const int* guard, int parts, BRed red) {
   if constexpr (UNIT) {
     alpha_zero = 0;
     alpha_one = 1;
     beta_zero = 1;
   }
+  constexpr int GR = 32 / KP;
+  constexpr bool kAhead = KP >= 16;  // a row's first entries are read a row ahead
+  const int lane = threadIdx.x & 31;
+  const int grp = lane / KP, j = lane % KP;
+  const bool on = j < k;
+  double dot[2] = {0.0, 0.0};
+  // The warp's rows, in order: those of share blockIdx.x and those of share
+  // blockIdx.x + gridDim.x (if there is one) by turns.
+  const int nv = (int)(blockIdx.x + gridDim.x) < parts ? 2 : 1;
+  const int64_t step = (int64_t)parts * kBWarps;
+  const int64_t first = (int64_t)(threadIdx.x >> 5) * parts + blockIdx.x;
+  auto rows_of = [&](int i) {
+    return first + (i & (nv - 1)) * (int64_t)gridDim.x + (i >> (nv - 1)) * step;
+  };
+  // The matrix does not change while a solve runs: with rows read ahead, the
+  // first row's entries and the second row's offsets come before the wait on
+  // the previous kernel.
+  int e1 = 0, len1 = 0, c1 = 0;  // the next row's extent; its entry of this lane
+  V v1 = V(0.0f);
+  auto extent = [&](int64_t w, int& e, int& l) {
+    const int64_t row = w * GR + grp;
+    e = l = 0;
+    if (row < nrow) {
+      e = __ldg(off + row);
+      l = __ldg(off + row + 1) - e;
+    }
+  };
+  auto entry = [&](int e, int l) {
+    c1 = 0;
+    v1 = V(0.0f);
+    if (j < l) {
+      c1 = __ldg(col + e + j);
+      v1 = __ldg(val + e + j);
+    }
+  };
+  int e2 = 0, len2 = 0;
+  if (kAhead && !alpha_zero) {
+    extent(rows_of(0), e1, len1);
+    extent(rows_of(1), e2, len2);
+    entry(e1, len1);
+  }
   pdl_wait();
   pdl_launch_dependents();
   if (guard_off(guard)) return;
-  constexpr int GR = 32 / KP;
-  const int lane = threadIdx.x & 31;
-  const int grp = lane / KP, j = lane % KP;
-  const int64_t warps_total = (int64_t)gridDim.x * kBWarps;
-  const bool on = j < k;
-  double dot = 0.0;
-  for (int64_t wb = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; wb * GR < nrow;
-       wb += warps_total) {
+  for (int i = 0;; ++i) {
+    const int64_t wb = rows_of(i);
+    if (wb * GR >= nrow) break;
     const int row = (int)(wb * GR) + grp;
     const bool live = row < nrow;
+    // What the row's end needs is read with its first entries (a dot with the
+    // output itself, red.w == Z, takes the value written).
+    const int64_t idx = (int64_t)row * k + j;
+    double wv = 0.0;
+    T x2 = T(0), wm_r = T(0);
+    if (on && live) {
+      if (DOT)
+        wv = (!std::is_same<T, double>::value && red.w_f64) ? ((const double*)red.w)[idx]
+                                                             : (double)((const T*)red.w)[idx];
+      if (EPI == BE_SQLAP_BWD && !alpha_zero) {
+        x2 = X2[idx];
+        wm_r = wm[row];
+      }
+    }
     T acc = T(0);
     if (!alpha_zero) {
       int e0 = 0, len = 0;
-      if (live) {
-        e0 = __ldg(off + row);
-        len = __ldg(off + row + 1) - e0;
+      int c_first = 0;
+      V v_first = V(0.0f);
+      if constexpr (kAhead) {
+        e0 = e1;
+        len = len1;
+        c_first = c1;
+        v_first = v1;
+        e1 = e2;
+        len1 = len2;
+        entry(e1, len1);
+        extent(rows_of(i + 2), e2, len2);
+      } else {
+        extent(wb, e0, len);
       }
       int maxlen = len;
 #pragma unroll
@@ -263,9 +374,9 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
         // Wide groups: enough independent work per warp already; one
         // entry at a time (the batched form measured slower and spills).
         for (int base = 0; base < maxlen; base += KP) {
-          int c_l = 0;
-          T v_l = T(0);
-          if (base + j < len) {
+          int c_l = c_first;
+          T v_l = cvt<T, V>(v_first);
+          if (base > 0 && base + j < len) {
             c_l = __ldg(col + e0 + base + j);
             v_l = cvt<T, V>(__ldg(val + e0 + base + j));
           }
@@ -306,12 +417,11 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
       }
     }
     if (on && live) {
-      const int64_t idx = (int64_t)row * k + j;
       T out;
       if (EPI == BE_SQLAP_BWD) {
         out = T(0);
         if (!alpha_zero) {
-          out = fma_bt<T>(wm[row], X2[idx], acc);
+          out = fma_bt<T>(wm_r, x2, acc);
           if (!alpha_one) out = (T)alpha * out;
         }
       } else {
@@ -320,14 +430,20 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
       if (!beta_zero) out = fma_bt<T>((T)beta, Y[idx], out);
       Z[idx] = out;
       if (DOT) {
-        const double wv = (!std::is_same<T, double>::value && red.w_f64)
-                              ? ((const double*)red.w)[idx]
-                              : (double)((const T*)red.w)[idx];
-        dot = fma((double)out, wv, dot);
+        // One FMA and two selects: an FP64 instruction costs the same when
+        // it is predicated off.
+        const double w = red.w == (const void*)Z ? (double)out : wv;
+        const bool second = (i & (nv - 1)) != 0;
+        const double sum = fma((double)out, w, second ? dot[1] : dot[0]);
+        dot[0] = second ? dot[0] : sum;
+        dot[1] = second ? sum : dot[1];
       }
     }
   }
-  if (DOT) b_reduce(red, b_fold<KP>(dot));
+  if (DOT) {
+    const double sums[2] = {b_fold<KP>(dot[0]), b_fold<KP>(dot[1])};
+    b_reduce(red, sums, nv, parts);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -352,39 +468,70 @@ bdot_kernel(int64_t n, int k, const T* a, const T* b, BRed red) {
       const int64_t row = wb * GR + grp;
       if (row < n) s = fma((double)a[row * k + j], (double)b[row * k + j], s);
     }
-  b_reduce(red, b_fold<KP>(s));
+  const double sums[1] = {b_fold<KP>(s)};
+  b_reduce(red, sums, 1, gridDim.x);
 }
 
 // X += alpha_j P; R -= alpha_j AP; reduce r.r  (inactive RHS untouched).
+// Bound by latency: each warp has kBUpdateRows rows in flight (the stores of a
+// row may alias the loads of the next as far as the compiler knows) and all
+// CTAs are resident, 14.3 us for 33^3 rows of 32 against 22.9 us with one row
+// at a time and CTAs for one and a third waves.
 // R32 != nullptr: also R32 = (float) R, the input of a float32
 // preconditioner inside the float64 loop.
 template <typename T, int KP>
-__global__ void __launch_bounds__(kBThreads)
+__global__ void __launch_bounds__(kBThreads, 2)
 bcg_update_kernel(int64_t n, int k, BatchScalars* bs, T* X, T* R, const T* P, const T* AP,
                   float* R32, BRed red) {
+  B_ROWS(KP);
+  constexpr int U = kBUpdateRows;
+  int64_t wb = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  T x[U], p[U];
+  // X and P are not written by the previous kernel (the product that wrote
+  // AP): the first rows of them are read before the wait.
+  auto read_xp = [&]() {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t row = (wb + u * warps_total) * GR + grp;
+      const bool in = row < n && j < k;
+      x[u] = in ? X[row * k + j] : T(0);
+      p[u] = in ? P[row * k + j] : T(0);
+    }
+  };
+  read_xp();
   pdl_wait();
   pdl_launch_dependents();
   if (*(volatile int*)&bs->any_active == 0) return;
-  B_ROWS(KP);
   const bool on = j < k && bs->active[j];
   const T a = on ? (T)bs->alpha[j] : T(0);
   double s = 0.0;
-  if (j < k)
-    for (int64_t wb = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x; wb * GR < n;
-         wb += warps_total) {
-      const int64_t row = wb * GR + grp;
-      if (row >= n) continue;
-      const int64_t idx = row * k + j;
-      T r = R[idx];
-      if (on) {
-        X[idx] = fma_bt<T>(a, P[idx], X[idx]);
-        r = fma_bt<T>(-a, AP[idx], r);
-        R[idx] = r;
-        if (R32) R32[idx] = (float)r;
-      }
-      s = fma((double)r, (double)r, s);
+  while (wb * GR < n) {
+    T r[U], w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t row = (wb + u * warps_total) * GR + grp;
+      const bool in = row < n && j < k;
+      r[u] = in ? R[row * k + j] : T(0);
+      w[u] = in && on ? AP[row * k + j] : T(0);
     }
-  b_reduce(red, b_fold<KP>(s));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t row = (wb + u * warps_total) * GR + grp;
+      if (row >= n || j >= k) continue;
+      const int64_t idx = row * k + j;
+      if (on) {
+        X[idx] = fma_bt<T>(a, p[u], x[u]);
+        r[u] = fma_bt<T>(-a, w[u], r[u]);
+        R[idx] = r[u];
+        if (R32) R32[idx] = (float)r[u];
+      }
+      s = fma((double)r[u], (double)r[u], s);
+    }
+    wb += U * warps_total;
+    if (wb * GR < n) read_xp();
+  }
+  const double sums[1] = {b_fold<KP>(s)};
+  b_reduce(red, sums, 1, gridDim.x);
 }
 
 // P = Z + beta_j P  (active RHS only); Z may be float32 (widened).
@@ -525,12 +672,13 @@ static void launch_bspmm(const BCsr& m, int k, const void* X, const void* Y, voi
   const int az = alpha == 0.0, a1 = alpha == 1.0, bz = beta == 0.0;
   with_kp(k, [&](auto kpc) {
     constexpr int KP = decltype(kpc)::value;
-    const int g = b_grid(m.nrow, KP);
+    const int parts = b_grid(m.nrow, KP);
+    const int g = std::min(parts, kBResidentCtas);
     auto go = [&](auto kern) {
       launch_k(kern, g, kBThreads, 0, st, m.nrow, k, (const int32_t*)m.off.as<int32_t>(),
                (const int32_t*)m.col.as<int32_t>(), (const V*)m.val.as<V>(), (const T*)X,
                (const T*)Y, (T*)Z, alpha, beta, az, a1, bz, (const T*)wm, (const T*)X2, guard,
-               red);
+               parts, red);
     };
     const bool unit = !az && a1 && bz;
     if (dot && dot->w) {
@@ -734,7 +882,7 @@ struct BSolver {
   template <typename T>
   int record_init(int k, const void* B, void* X, cudaStream_t st) {
     int rc;
-    GBPC_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned int), st));
+    GBPC_CUDA_TRY(cudaMemsetAsync(counter.p, 0, sizeof(unsigned int) * (1 + kBGroups), st));
     BRed rbb = red(B, BF_BB);
     with_kp(k, [&](auto kpc) {
       constexpr int KP = decltype(kpc)::value;
@@ -771,7 +919,7 @@ struct BSolver {
     float* r32 = mixed_m ? R32.as<float>() : nullptr;
     with_kp(k, [&](auto kpc) {
       constexpr int KP = decltype(kpc)::value;
-      launch_k(bcg_update_kernel<T, KP>, b_grid(n, KP), kBThreads, 0, st, n, k, S(), (T*)X,
+      launch_k(bcg_update_kernel<T, KP>, std::min(b_grid(n, KP), kBResidentCtas), kBThreads, 0, st, n, k, S(), (T*)X,
                (T*)R.p, (const T*)P.p, (const T*)AP.p, r32, rr);
     });
     GBPC_CUDA_TRY(cudaGetLastError());
@@ -1109,10 +1257,10 @@ extern "C" int gbpc_bsolver_create(gbpc_bop* A, gbpc_bop* M, int unroll, int max
   if (!rc && mixed_m) rc = s.R32.alloc(sizeof(float) * std::max<int64_t>(s.n, 1) * max_rhs);
   if (!rc && mixed_m) rc = s.Z32.alloc(sizeof(float) * std::max<int64_t>(s.n, 1) * max_rhs);
   if (!rc) rc = s.bs.alloc(sizeof(BatchScalars));
-  if (!rc) rc = s.partials.alloc(sizeof(double) * kBMaxCtas * kB);
-  if (!rc) rc = s.counter.alloc(sizeof(unsigned int));
+  if (!rc) rc = s.partials.alloc(sizeof(double) * (kBMaxCtas + kBGroups) * kB);
+  if (!rc) rc = s.counter.alloc(sizeof(unsigned int) * (1 + kBGroups));
   if (!rc && (cudaMemsetAsync(s.bs.p, 0, sizeof(BatchScalars), (cudaStream_t)stream) != cudaSuccess ||
-              cudaMemsetAsync(s.counter.p, 0, sizeof(unsigned int), (cudaStream_t)stream) != cudaSuccess))
+              cudaMemsetAsync(s.counter.p, 0, sizeof(unsigned int) * (1 + kBGroups), (cudaStream_t)stream) != cudaSuccess))
     rc = GBPC_ERR_CUDA;
   if (rc) {
     delete h;
