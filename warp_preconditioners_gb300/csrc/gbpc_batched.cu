@@ -157,6 +157,7 @@ __device__ __forceinline__ void b_finalize(const BRed& red, int j, double total,
 // every other SM was idle; spread over 16 warps of different CTAs it takes a
 // chain of 38 adds on each.
 constexpr int kBGroups = 16;
+static_assert(kBGroups == kBWarps, "the last CTA adds a group to a warp");
 
 __device__ __forceinline__ void b_hand_in(const BRed& red, double s, unsigned part,
                                           unsigned parts) {
@@ -221,10 +222,17 @@ __device__ __forceinline__ void b_hand_in(const BRed& red, double s, unsigned pa
   if (lane == 0) *red.counter = 0u;
 }
 
+// Up to this many partial sums the last CTA adds all of them, a group to a
+// warp, in the same order: the 16 groups' second round of fence and counter
+// (1.3 us) costs more than the adds do on one SM.  A solve of 10^3 rows with
+// 16 right-hand sides (32 partial sums) takes 4.7 ms this way and 5.2 ms with
+// the groups on several CTAs; the costs cross near 200 partial sums.
+constexpr unsigned kBOneCta = 160;
+
 // Every thread calls this with its lane's sums: of partial sum blockIdx.x
 // and, with n == 2, of partial sum blockIdx.x + gridDim.x.  Warps are reduced
 // through shared memory in index order.  Nothing follows in the calling
-// kernels, so the other warps leave at once.
+// kernels, so warps without work leave at once.
 template <int N>
 __device__ __forceinline__ void b_reduce(const BRed& red, const double (&v)[N], int n,
                                          unsigned parts) {
@@ -233,10 +241,57 @@ __device__ __forceinline__ void b_reduce(const BRed& red, const double (&v)[N], 
 #pragma unroll
   for (int h = 0; h < N; ++h) sm[h][warp][lane] = v[h];
   __syncthreads();
-  if (warp >= n) return;
-  double s = sm[warp][0][lane];
+  const bool one = parts <= kBOneCta;  // then n == 1
+  if (warp >= n && !one) return;
+  double s = 0.0;
+  if (warp < n) {
+    s = sm[warp][0][lane];
 #pragma unroll
-  for (int w = 1; w < kBWarps; ++w) s += sm[warp][w][lane];
+    for (int w = 1; w < kBWarps; ++w) s += sm[warp][w][lane];
+  }
+  if (one) {
+    __shared__ bool last;
+    if (warp == 0) {
+      red.partials[(size_t)blockIdx.x * kB + lane] = s;
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) last = atomicAdd(red.counter, 1u) == parts - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double rz = 0.0;
+    int active = 0;
+    if (warp == 0 && red.bs) {
+      rz = red.bs->rz[lane];
+      active = red.bs->active[lane];
+    }
+    constexpr int L = (kBOneCta + kBGroups - 1) / kBGroups;
+    double p[L];
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      const unsigned c = warp + q * kBGroups;
+      p[q] = c < parts ? __ldcg(red.partials + (size_t)c * kB + lane) : 0.0;
+    }
+    s = 0.0;
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      if (warp + q * kBGroups >= parts) break;
+      s += p[q];
+    }
+    sm[0][warp][lane] = s;
+    __syncthreads();
+    if (warp != 0) return;
+    double total = sm[0][0][lane];
+#pragma unroll
+    for (int w = 1; w < kBGroups; ++w) {
+      if (w >= parts) break;
+      total += sm[0][w][lane];
+    }
+    b_finalize(red, lane, total, rz, active);
+    if (lane == 0) *red.counter = 0u;
+    return;
+  }
   b_hand_in(red, s, blockIdx.x + warp * gridDim.x, parts);
 }
 
@@ -317,10 +372,13 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
     const bool live = row < nrow;
     // What the row's end needs is read with its first entries (a dot with the
     // output itself, red.w == Z, takes the value written).
+    // Not for narrow groups: a warp has so many rows there that their chunks
+    // hide the loads, and the registers cost more (2 right-hand sides: 2 %).
+    constexpr bool kEarly = KP >= 4;
     const int64_t idx = (int64_t)row * k + j;
     double wv = 0.0;
     T x2 = T(0), wm_r = T(0);
-    if (on && live) {
+    auto operands = [&]() {
       if (DOT)
         wv = (!std::is_same<T, double>::value && red.w_f64) ? ((const double*)red.w)[idx]
                                                              : (double)((const T*)red.w)[idx];
@@ -328,7 +386,8 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
         x2 = X2[idx];
         wm_r = wm[row];
       }
-    }
+    };
+    if (kEarly && on && live) operands();
     T acc = T(0);
     if (!alpha_zero) {
       int e0 = 0, len = 0;
@@ -354,7 +413,11 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
       // stop at the chunk's last entry in any row of the warp (a uniform
       // exit): an FP64 instruction costs its full issue slot even with every
       // lane predicated off.
-      if constexpr (KP == 1) {
+      if constexpr (KP <= 2) {
+        // Narrow groups: every lane reads its row's entries itself, four at a
+        // time (a pair at a time and by shuffles, a solve with 2 right-hand
+        // sides takes 8.4 ms against 6.6 ms at 12^3 rows, 74.9 against 69.6
+        // at 32^3).
         constexpr int U = 4;
         for (int base = 0; base < maxlen; base += U) {
           T xv[U], vv[U];
@@ -362,7 +425,7 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
           for (int e = 0; e < U; ++e) {
             const bool in = base + e < len;
             vv[e] = in ? cvt<T, V>(__ldg(val + e0 + base + e)) : T(0);
-            xv[e] = in ? X[(int64_t)__ldg(col + e0 + base + e) * k] : T(0);
+            xv[e] = in && on ? X[(int64_t)__ldg(col + e0 + base + e) * k + j] : T(0);
           }
 #pragma unroll
           for (int e = 0; e < U; ++e) {
@@ -417,6 +480,7 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
       }
     }
     if (on && live) {
+      if (!kEarly) operands();
       T out;
       if (EPI == BE_SQLAP_BWD) {
         out = T(0);
@@ -441,7 +505,8 @@ bspmm_kernel(int nrow, int k, const int32_t* __restrict__ off, const int32_t* __
     }
   }
   if (DOT) {
-    const double sums[2] = {b_fold<KP>(dot[0]), b_fold<KP>(dot[1])};
+    double sums[2] = {b_fold<KP>(dot[0]), 0.0};
+    if (nv == 2) sums[1] = b_fold<KP>(dot[1]);
     b_reduce(red, sums, nv, parts);
   }
 }
@@ -484,7 +549,7 @@ __global__ void __launch_bounds__(kBThreads, 2)
 bcg_update_kernel(int64_t n, int k, BatchScalars* bs, T* X, T* R, const T* P, const T* AP,
                   float* R32, BRed red) {
   B_ROWS(KP);
-  constexpr int U = kBUpdateRows;
+  constexpr int U = KP >= 4 ? kBUpdateRows : 1;  // narrow groups: a warp has 16 or 32 rows anyway
   int64_t wb = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   T x[U], p[U];
   // X and P are not written by the previous kernel (the product that wrote
@@ -516,6 +581,8 @@ bcg_update_kernel(int64_t n, int k, BatchScalars* bs, T* X, T* R, const T* P, co
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
+      // A uniform exit: predicated FP64 instructions are not free.
+      if ((wb + u * warps_total) * GR >= n) break;
       const int64_t row = (wb + u * warps_total) * GR + grp;
       if (row >= n || j >= k) continue;
       const int64_t idx = row * k + j;
