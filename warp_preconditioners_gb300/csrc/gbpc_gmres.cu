@@ -4,8 +4,8 @@
 // lifted-biharmonic and indefinite call sites use (tests/test_biharmonic.py:32,
 // tests/test_indefinite.py:130, benchmarks/indefinite.py:192-225).  Its exact
 // iterates are not pinned by the reference; this is the textbook method:
-// Arnoldi on A M with classical Gram-Schmidt applied twice (each pass one
-// multi-dot and one multi-axpy over the basis), Givens rotations on the
+// Arnoldi on A M with classical Gram-Schmidt applied twice (the first pass's
+// multi-axpy and the second's multi-dot read the basis together), Givens rotations on the
 // Hessenberg column, the residual norm |g_{j+1}| as the stopping quantity
 // (stop when it is <= max(atol, tol |b|) or after maxiter steps), and at the
 // end of a cycle x += M (V y) with H y = g solved by back-substitution.
@@ -14,7 +14,8 @@
 // conditional while-node whose body is one Arnoldi step followed by a
 // conditional if-node holding the end-of-cycle update (back-substitution,
 // solution update, new residual).  Every reduction is deterministic: per-CTA
-// partials, combined in a fixed order by the last CTA to finish.
+// partials, combined in a fixed order by the last CTA to finish or, in the
+// Arnoldi step, by every CTA of the kernel that uses the sum.
 //
 // FP64 throughput, not memory, bounds the Gram-Schmidt kernels on this part
 // (about 1.7 FP64 operations per clock per SM, the same for a warp
@@ -49,17 +50,21 @@ constexpr int kGCluster = 8;      // CTAs per cluster of the multi-dot
 constexpr int kMdotCtas = 152 * 2;  // multi-dot CTAs (at most; a multiple of kGCluster)
 constexpr int kMdotClusters = kMdotCtas / kGCluster;
 static_assert(kMdotCtas % kGCluster == 0, "multi-dot grid must hold whole clusters");
-static_assert(kMdotClusters <= kGCtas, "multi-dot partials fit the partials buffer");
+// A step's sums in the partials buffer: of the two multi-dots
+// ([cluster][kGMaxK]) and of the norm ([CTA]).
+constexpr size_t kDotParts = (size_t)kMdotClusters * kGMaxK;
+static_assert(2 * kDotParts + kGCtas <= (size_t)kGCtas * kGMaxK,
+              "a step's sums fit the partials buffer");
 
 struct GmresState {
-  int m, j, it, maxiter;
+  int m, j, jn, it, maxiter;  // j: column of the step, jn: of the next one
   int done, not_done, restart, resid;  // flags (ints: operator guards point at them)
   double tol, atol, atol_sq, bb, beta2, ww, res, inv;
   unsigned long long while_handle, if_handle;
 };
 
-// Hessenberg workspace: H column-major (m+1) x m, rotations, g, y, the
-// current column and the coefficients of the last Gram-Schmidt pass.
+// Hessenberg workspace: H column-major (m+1) x m, rotations, g, y and the
+// current column.
 struct GmresWork {
   double* H;
   double* cs;
@@ -67,7 +72,6 @@ struct GmresWork {
   double* g;
   double* y;
   double* hcol;
-  double* coef;
 };
 
 __device__ __forceinline__ void set_cond(unsigned long long h, bool v) {
@@ -129,6 +133,7 @@ __global__ void gm_setup_kernel(GmresState* s, int m, double tol, double atol, i
                                 unsigned long long while_handle, unsigned long long if_handle) {
   s->m = m;
   s->j = 0;
+  s->jn = 0;
   s->it = 0;
   s->maxiter = maxiter;
   s->done = 0;
@@ -199,21 +204,67 @@ __device__ __forceinline__ double scatter_sum(const double (&a)[C]) {
   return t;
 }
 
-// One pass over the rows for basis vectors i0 .. i0 + C - 1 (C independent
-// loads per row), leaving each warp's sums in sm[warp][i0 + c].
+// v - sum_q cf[q] V_{i0+q}[r] for C basis vectors, loads issued together,
+// FMAs in basis order.
 template <int C>
-__device__ __forceinline__ void mdot_pass(int64_t n, const double* __restrict__ V,
-                                          const double* __restrict__ w, int i0,
-                                          double (*sm)[kGMaxK]) {
+__device__ __forceinline__ double update_pass(double v, const double* __restrict__ Vi, int64_t n,
+                                              int64_t r, const double* cf) {
+  double t[C];
+#pragma unroll
+  for (int q = 0; q < C; ++q) t[q] = Vi[(size_t)q * n + r];
+#pragma unroll
+  for (int q = 0; q < C; ++q) v = fma(-cf[q], t[q], v);
+  return v;
+}
+
+template <int C>
+__device__ __forceinline__ double update_rest(int rem, double v, const double* Vi, int64_t n,
+                                              int64_t r, const double* cf) {
+  if constexpr (C > 0) {
+    if (rem == C) return update_pass<C>(v, Vi, n, r, cf);
+    return update_rest<C - 1>(rem, v, Vi, n, r, cf);
+  }
+  return v;
+}
+
+// One pass over the rows for basis vectors i0 .. i0 + C - 1 (C independent
+// loads per row), leaving each warp's sums in sm[warp][i0 + c].  UPDATE: w
+// loses cf[i] V_i for i < i0 + C first, so i0 + C is the whole basis.
+template <int C, bool UPDATE>
+__device__ __forceinline__ void mdot_pass(int64_t n, const double* __restrict__ V, double* w,
+                                          int i0, const double* cf, double (*sm)[kGMaxK]) {
   double acc[C];
 #pragma unroll
   for (int q = 0; q < C; ++q) acc[q] = 0.0;
   const double* Vi = V + (size_t)i0 * n;
-  for (int64_t r = (int64_t)blockIdx.x * kGT + threadIdx.x; r < n; r += (int64_t)gridDim.x * kGT) {
-    const double wr = w[r];
+  const int64_t step = (int64_t)gridDim.x * kGT;
+  int64_t r = (int64_t)blockIdx.x * kGT + threadIdx.x;
+  if constexpr (!UPDATE) {  // two rows' loads in flight
+    for (; r + step < n; r += 2 * step) {
+      const double w0 = w[r], w1 = w[r + step];
+      double t[2 * C];
+#pragma unroll
+      for (int q = 0; q < C; ++q) {
+        t[q] = Vi[(size_t)q * n + r];
+        t[C + q] = Vi[(size_t)q * n + r + step];
+      }
+#pragma unroll
+      for (int q = 0; q < C; ++q) acc[q] = fma(t[C + q], w1, fma(t[q], w0, acc[q]));
+    }
+  }
+  for (; r < n; r += step) {
+    double wr = w[r];
+    if (UPDATE)
+      for (int i = 0; i < i0; i += kGChunk)
+        wr = update_pass<kGChunk>(wr, V + (size_t)i * n, n, r, cf + i);
     double t[C];
 #pragma unroll
     for (int q = 0; q < C; ++q) t[q] = Vi[(size_t)q * n + r];
+    if (UPDATE) {
+#pragma unroll
+      for (int q = 0; q < C; ++q) wr = fma(-cf[i0 + q], t[q], wr);
+      w[r] = wr;
+    }
 #pragma unroll
     for (int q = 0; q < C; ++q) acc[q] = fma(t[q], wr, acc[q]);
   }
@@ -223,23 +274,67 @@ __device__ __forceinline__ void mdot_pass(int64_t n, const double* __restrict__ 
   if ((lane & ((1 << low) - 1)) == 0 && c < C) sm[threadIdx.x >> 5][i0 + c] = total;
 }
 
-// The last rem (< 16) basis vectors with a pass of exactly that width.
-template <int C>
-__device__ __forceinline__ void mdot_rest(int rem, int64_t n, const double* V, const double* w,
-                                          int i0, double (*sm)[kGMaxK]) {
+// The last rem (1 .. 16) basis vectors with a pass of exactly that width.
+template <int C, bool UPDATE>
+__device__ __forceinline__ void mdot_rest(int rem, int64_t n, const double* V, double* w, int i0,
+                                          const double* cf, double (*sm)[kGMaxK]) {
   if constexpr (C > 0) {
-    if (rem == C) mdot_pass<C>(n, V, w, i0, sm);
-    else mdot_rest<C - 1>(rem, n, V, w, i0, sm);
+    if (rem == C) mdot_pass<C, UPDATE>(n, V, w, i0, cf, sm);
+    else mdot_rest<C - 1, UPDATE>(rem, n, V, w, i0, cf, sm);
   }
 }
 
-// coef[i] = V_i . w for i <= j (this pass); hcol accumulates the passes.
-// Warp sums (scatter_sum) -> CTA sums -> cluster sums in the cluster's
-// first CTA, read through distributed shared memory -> per-cluster partials
-// -> the last cluster to finish adds them, one coefficient per lane.
-__global__ void __cluster_dims__(kGCluster, 1, 1) __launch_bounds__(kGT)
-gm_mdot_kernel(int64_t n, const double* V, const double* w, GmresState* s, GmresWork wk,
-               int accumulate, double* partials, unsigned int* counter) {
+// cf[i] = sum of the clusters' partials of coefficient i < k, by the whole
+// CTA: thread (g, i) adds clusters g, g + 8, ... of coefficient i, then one
+// thread a coefficient adds the eight sums.  The threads are numbered without
+// gaps: every CTA does this, and an FP64 warp instruction costs the same
+// whatever its active lanes.
+__device__ __forceinline__ void coefficients(const double* partials, unsigned clusters, int k,
+                                             double (*sm)[kGMaxK], double* cf) {
+  constexpr int G = kGT / 32, L = (kMdotClusters + G - 1) / G;
+  for (int e = threadIdx.x; e < G * k; e += kGT) {
+    const unsigned g = e / k;
+    const int i = e - (int)g * k;
+    double v[L];
+#pragma unroll
+    for (int q = 0; q < L; ++q) {
+      const unsigned c = g + q * G;
+      v[q] = c < clusters ? __ldcg(partials + (size_t)c * kGMaxK + i) : 0.0;
+    }
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < L; ++q) t += v[q];
+    sm[g][i] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < k) {
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < G; ++q) t += sm[q][threadIdx.x];
+    cf[threadIdx.x] = t;
+  }
+  __syncthreads();
+}
+
+// Sums of V_i . w for i <= j, per cluster, for the kernel that uses them.
+// Warp sums (scatter_sum) -> CTA sums -> cluster sums in the cluster's first
+// CTA, read through distributed shared memory.
+//
+// UPDATE (second Gram-Schmidt pass): the first pass's coefficients are added
+// up from `in` and w loses its projection before the dot products, so the
+// two read the basis once; basis vectors before the last chunk of 16 are read
+// again, by the thread and CTA that read them for the update.  The first
+// pass's kernel sets j.  Bound by FP64 issue (one multiply-add an entry of
+// the basis, two with UPDATE, and the butterfly) and by the latency of the
+// few rows a thread has, so two rows are read at once.  62 GMRES(31) steps
+// (GB300): 17^3 tet cube 5.39 -> 5.05 ms, 40^3 (128,000 unknowns) 8.11 -> 7.31,
+// 70^3 18.4 -> 17.6 against four passes over the basis whose last CTAs
+// finish each sum; with the update and the dot products kept apart and only
+// the sums moved, 70^3 took 0.7 ms more than before.
+template <bool UPDATE>
+__global__ void __cluster_dims__(kGCluster, 1, 1) __launch_bounds__(kGT, kMdotCtas / kSms)
+gm_mdot_kernel(int64_t n, const double* V, double* w, GmresState* s, GmresWork wk, const double* in,
+               double* out) {
   pdl_wait();
   pdl_launch_dependents();
   // Uniform over the grid (nothing writes it during this kernel), so a whole
@@ -247,11 +342,18 @@ gm_mdot_kernel(int64_t n, const double* V, const double* w, GmresState* s, Gmres
   if (*(volatile int*)&s->not_done == 0) return;
   __shared__ double sm[kGT / 32][kGMaxK];
   __shared__ double cta[kGMaxK];
-  const int k = s->j + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int i0 = 0;
-  for (; i0 + kGChunk <= k; i0 += kGChunk) mdot_pass<kGChunk>(n, V, w, i0, sm);
-  mdot_rest<kGChunk - 1>(k - i0, n, V, w, i0, sm);
+  const int j = UPDATE ? s->j : s->jn, k = j + 1;
+  if (UPDATE) {
+    // `cta` holds the coefficients until the CTA's sums replace them.
+    coefficients(in, gridDim.x / kGCluster, k, sm, cta);
+    if (blockIdx.x == 0 && threadIdx.x < k) wk.hcol[threadIdx.x] = cta[threadIdx.x];
+  } else if (blockIdx.x == 0 && threadIdx.x == 0) {
+    s->j = j;  // no CTA of this kernel reads it
+  }
+  const int rem = (k - 1) % kGChunk + 1, last = k - rem;
+  mdot_rest<kGChunk, UPDATE>(rem, n, V, w, last, cta, sm);
+  for (int i0 = 0; i0 < last; i0 += kGChunk)
+    mdot_pass<kGChunk, false>(n, V, w, i0, nullptr, sm);
   __syncthreads();
   if (threadIdx.x < k) {
     double t = 0.0;
@@ -261,45 +363,19 @@ gm_mdot_kernel(int64_t n, const double* V, const double* w, GmresState* s, Gmres
   }
   cg::cluster_group cluster = cg::this_cluster();
   cluster.sync();
-  const bool leader = cluster.block_rank() == 0;
-  if (leader && threadIdx.x < k) {
+  if (cluster.block_rank() == 0 && threadIdx.x < k) {
     double v[kGCluster];
 #pragma unroll
     for (int q = 0; q < kGCluster; ++q) v[q] = cluster.map_shared_rank(cta, q)[threadIdx.x];
     double t = 0.0;
 #pragma unroll
     for (int q = 0; q < kGCluster; ++q) t += v[q];
-    partials[(size_t)(blockIdx.x / kGCluster) * kGMaxK + threadIdx.x] = t;
+    out[(size_t)(blockIdx.x / kGCluster) * kGMaxK + threadIdx.x] = t;
   }
   cluster.sync();  // the leader's remote reads are done before any CTA exits
-  if (!leader) return;
-  const unsigned nc = gridDim.x / kGCluster;
-  if (arrive_last(counter, nc)) {
-    // Warp w adds clusters w, w + 8, ... for coefficients lane, lane + 32, ...
-    constexpr int L = (kMdotClusters + kGT / 32 - 1) / (kGT / 32);
-    for (int i = lane; i < k; i += 32) {
-      double v[L];
-#pragma unroll
-      for (int q = 0; q < L; ++q) {
-        const unsigned c = warp + q * (kGT / 32);
-        v[q] = c < nc ? __ldcg(partials + (size_t)c * kGMaxK + i) : 0.0;
-      }
-      double t = 0.0;
-#pragma unroll
-      for (int q = 0; q < L; ++q) t += v[q];
-      sm[warp][i] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x < k) {
-      double t = 0.0;
-#pragma unroll
-      for (int q = 0; q < kGT / 32; ++q) t += sm[q][threadIdx.x];
-      wk.coef[threadIdx.x] = t;
-      wk.hcol[threadIdx.x] = accumulate ? wk.hcol[threadIdx.x] + t : t;
-    }
-    if (threadIdx.x == 0) *counter = 0u;
-  }
 }
+
+__device__ __forceinline__ bool breaks_down(double hn) { return !(hn > 0.0) || !isfinite(hn); }
 
 // Givens update of column j and the stopping test, by one full warp.
 // Applying rotations 0..j-1 to the new column is the affine recurrence
@@ -360,11 +436,11 @@ __device__ void gm_step_finalize(GmresState* s, GmresWork wk, double ww) {
   wk.g[j] = c * gj;
   s->res = fabs(wk.g[j + 1]);
   s->it += 1;
-  const bool breakdown = !(hn > 0.0) || !isfinite(hn);
-  s->inv = breakdown ? 0.0 : 1.0 / hn;
+  const bool breakdown = breaks_down(hn);
   const bool conv = s->res * s->res <= s->atol_sq;
   const bool stop = conv || s->it >= s->maxiter;
   const bool restart = stop || breakdown || (j + 1 == m);
+  s->jn = j + 1;
   s->done = stop;
   s->not_done = !stop;
   s->restart = restart;
@@ -373,41 +449,19 @@ __device__ void gm_step_finalize(GmresState* s, GmresWork wk, double ww) {
   set_cond(s->while_handle, !stop);
 }
 
-// v - sum_q cf[q] V_{i0+q}[r] for C basis vectors, loads issued together,
-// FMAs in basis order.
-template <int C>
-__device__ __forceinline__ double update_pass(double v, const double* __restrict__ Vi, int64_t n,
-                                              int64_t r, const double* cf) {
-  double t[C];
-#pragma unroll
-  for (int q = 0; q < C; ++q) t[q] = Vi[(size_t)q * n + r];
-#pragma unroll
-  for (int q = 0; q < C; ++q) v = fma(-cf[q], t[q], v);
-  return v;
-}
-
-template <int C>
-__device__ __forceinline__ double update_rest(int rem, double v, const double* Vi, int64_t n,
-                                              int64_t r, const double* cf) {
-  if constexpr (C > 0) {
-    if (rem == C) return update_pass<C>(v, Vi, n, r, cf);
-    return update_rest<C - 1>(rem, v, Vi, n, r, cf);
-  }
-  return v;
-}
-
-// w -= sum_i coef[i] V_i; with `norm`, ww = w.w and the step finalize.
-__global__ void __launch_bounds__(kGT)
-gm_update_kernel(int64_t n, const double* V, double* w, GmresState* s, GmresWork wk, int norm,
-                 double* partials, unsigned int* counter) {
+// w -= sum_i coef[i] V_i with the second pass's coefficients, which are added
+// up here; the last CTA adds w.w and takes 1 / |w| (0 at a breakdown).
+__global__ void __launch_bounds__(kGT, kGCtas / kSms)
+gm_update_kernel(int64_t n, const double* V, double* w, GmresState* s, GmresWork wk,
+                 const double* in, unsigned clusters, double* norms, unsigned int* counter) {
   pdl_wait();
   pdl_launch_dependents();
   if (*(volatile int*)&s->not_done == 0) return;
-  __shared__ double sm[kGT / 32];
+  __shared__ double sm[kGT / 32][kGMaxK];
   __shared__ double cf[kGMaxK];
   const int k = s->j + 1;
-  if (threadIdx.x < k) cf[threadIdx.x] = wk.coef[threadIdx.x];
-  __syncthreads();
+  coefficients(in, clusters, k, sm, cf);
+  if (blockIdx.x == 0 && threadIdx.x < k) wk.hcol[threadIdx.x] += cf[threadIdx.x];
   double acc = 0.0;
   for (int64_t r = (int64_t)blockIdx.x * kGT + threadIdx.x; r < n; r += (int64_t)gridDim.x * kGT) {
     double v = w[r];
@@ -418,30 +472,32 @@ gm_update_kernel(int64_t n, const double* V, double* w, GmresState* s, GmresWork
     w[r] = v;
     acc = fma(v, v, acc);
   }
-  if (!norm) return;
-  const double c = cta_sum(acc, sm);
-  if (threadIdx.x == 0) partials[blockIdx.x] = c;
+  const double c = cta_sum(acc, sm[0]);
+  if (threadIdx.x == 0) norms[blockIdx.x] = c;
   if (arrive_last(counter, gridDim.x)) {
-    const double t = cta_total(partials, gridDim.x, sm);
-    if (threadIdx.x < 32) {
-      const double ww = __shfl_sync(0xffffffffu, t, 0);
-      if (threadIdx.x == 0) {
-        s->ww = ww;
-        *counter = 0u;
-      }
-      gm_step_finalize(s, wk, ww);
+    const double t = cta_total(norms, gridDim.x, sm[0]);
+    if (threadIdx.x == 0) {
+      const double hn = sqrt(t);
+      s->ww = t;
+      s->inv = breaks_down(hn) ? 0.0 : 1.0 / hn;
+      *counter = 0u;
     }
   }
 }
 
-// v_{j+1} = w / h_{j+1} into the basis and the fixed current vector, then j++
-// (the last CTA, after every CTA has read j).
+// v_{j+1} = w / h_{j+1} into the basis and the fixed current vector.  CTA 0
+// also ends the step (Givens, flags, jn) while the others write; in the
+// update's last CTA that chain of roots and divisions had the chip to itself.
+// No other CTA reads what it changes but for not_done, which turns 0 only
+// after the last step, whose v_{j+1} nothing uses (nor is it used when a
+// cycle ends).  The other threads take no root or division (the update left
+// 1 / |w|): with one each, this kernel was FP64-bound and 62 steps at 40^3
+// took 8.2 ms.
 __global__ void __launch_bounds__(kGT)
-gm_next_kernel(int64_t n, double* V, const double* w, double* vcur, GmresState* s,
-               unsigned int* counter) {
+gm_next_kernel(int64_t n, double* V, const double* w, double* vcur, GmresState* s, GmresWork wk) {
   pdl_wait();
   pdl_launch_dependents();
-  if (*(volatile int*)&s->restart != 0 || *(volatile int*)&s->not_done == 0) return;
+  if (*(volatile int*)&s->not_done == 0) return;
   const int j1 = s->j + 1;
   const double inv = s->inv;
   double* Vn = V + (size_t)j1 * n;
@@ -450,10 +506,7 @@ gm_next_kernel(int64_t n, double* V, const double* w, double* vcur, GmresState* 
     Vn[r] = v;
     vcur[r] = v;
   }
-  if (arrive_last(counter, gridDim.x) && threadIdx.x == 0) {
-    s->j = j1;
-    *counter = 0u;
-  }
+  if (blockIdx.x == 0 && threadIdx.x < 32) gm_step_finalize(s, wk, s->ww);
 }
 
 // End of a cycle: H y = g by back-substitution, one warp.  Column-oriented:
@@ -519,6 +572,7 @@ __global__ void gm_begin_kernel(GmresState* s, GmresWork wk) {
   wk.g[0] = beta;
   s->res = beta;
   s->j = 0;
+  s->jn = 0;
   const bool conv = s->beta2 <= s->atol_sq;
   const bool stop = conv || !(beta > 0.0) || !isfinite(beta) || s->it >= s->maxiter;
   s->inv = stop ? 0.0 : 1.0 / beta;
@@ -582,10 +636,9 @@ struct Gmres {
     wk.g = wk.sn + m;
     wk.y = wk.g + (m + 1);
     wk.hcol = wk.y + m;
-    wk.coef = wk.hcol + (m + 1);
     return wk;
   }
-  static size_t work_doubles(int m) { return (size_t)(m + 1) * m + 2 * (size_t)m + 2 * (size_t)(m + 1) + m + (m + 1); }
+  static size_t work_doubles(int m) { return (size_t)(m + 1) * m + 2 * (size_t)m + 2 * (size_t)(m + 1) + m; }
 
   int precondition(const double* in, double* out, const int* guard, cudaStream_t st) {
     if (M) return M->apply(in, nullptr, out, 1.0, 0.0, guard, nullptr, st);
@@ -627,17 +680,20 @@ struct Gmres {
       in = t.as<double>();
     }
     if ((rc = A->apply(in, nullptr, w.p, 1.0, 0.0, guard, nullptr, st))) return rc;
-    for (int pass = 0; pass < 2; ++pass) {
-      GBPC_CUDA_TRY(launch_k(gm_mdot_kernel, mdot_grid(n), kGT, 0, st, n,
-                             (const double*)V.as<double>(), (const double*)w.as<double>(), S(), W(),
-                             pass, partials.as<double>(), counter.as<unsigned int>()));
-      GBPC_CUDA_TRY(launch_k(gm_update_kernel, g_grid(n), kGT, 0, st, n,
-                             (const double*)V.as<double>(), w.as<double>(), S(), W(), pass,
-                             partials.as<double>(), counter.as<unsigned int>()));
-    }
-    GBPC_CUDA_TRY(launch_k(gm_next_kernel, g_grid(n), kGT, 0, st, n, V.as<double>(),
-                           (const double*)w.as<double>(), vcur.as<double>(), S(),
+    const double* basis = V.as<double>();
+    double* dots = partials.as<double>();
+    double* dots2 = dots + kDotParts;
+    double* norms = dots2 + kDotParts;
+    const int grid = mdot_grid(n);
+    GBPC_CUDA_TRY(launch_k(gm_mdot_kernel<false>, grid, kGT, 0, st, n, basis, w.as<double>(), S(),
+                           W(), (const double*)nullptr, dots));
+    GBPC_CUDA_TRY(launch_k(gm_mdot_kernel<true>, grid, kGT, 0, st, n, basis, w.as<double>(), S(),
+                           W(), (const double*)dots, dots2));
+    GBPC_CUDA_TRY(launch_k(gm_update_kernel, g_grid(n), kGT, 0, st, n, basis, w.as<double>(), S(),
+                           W(), (const double*)dots2, (unsigned)(grid / kGCluster), norms,
                            counter.as<unsigned int>()));
+    GBPC_CUDA_TRY(launch_k(gm_next_kernel, g_grid(n), kGT, 0, st, n, V.as<double>(),
+                           (const double*)w.as<double>(), vcur.as<double>(), S(), W()));
     return GBPC_OK;
   }
 
