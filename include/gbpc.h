@@ -221,6 +221,12 @@ int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int32_t* g_col
                  const void* g_val, const int32_t* gt_off, const int32_t* gt_col,
                  const void* gt_val, int value_dtype, int vector_dtype, void* stream,
                  gbpc_op** out);
+/* The same for two interleaved vectors, z = alpha (G^T G (x) I_2) x + beta y,
+ * from the scalar G and G^T: what gbpc_op_fsai gives for the 2 x 2 blocks
+ * g I_2 (RepeatedFSAI, warp_preconditioners/biharmonic.py). */
+int gbpc_op_fsai_pair(int nrow, const int32_t* g_off, const int32_t* g_col, const void* g_val,
+                      const int32_t* gt_off, const int32_t* gt_col, const void* gt_val,
+                      int value_dtype, int vector_dtype, void* stream, gbpc_op** out);
 /* New values of G and G^T (same patterns as at creation) for an FSAI
  * operator, written in place so that captured applies use them (the
  * reference's refit keeps G.values and GT.values pointers). */

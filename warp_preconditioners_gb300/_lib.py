@@ -68,6 +68,7 @@ _SIGNATURES = {
     "gbpc_op_sparse": [_int, _int, _int, _vp, _vp, _vp, _int, _int, _vp, ctypes.POINTER(_vp)],
     "gbpc_op_fsai": [_int, _int, _vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _vp,
                      ctypes.POINTER(_vp)],
+    "gbpc_op_fsai_pair": [_int, _vp, _vp, _vp, _vp, _vp, _vp, _int, _int, _vp, ctypes.POINTER(_vp)],
     "gbpc_op_sqlap": [_int, _vp, _vp, _vp, _int, _vp, _vp, _int, _dbl, _vp, ctypes.POINTER(_vp)],
     "gbpc_sqlap_rhs": [_vp, _vp, _vp, _vp],
     "gbpc_op_diagonal": [_int, _int, _vp, _vp, _vp, _int, _vp, ctypes.POINTER(_vp)],

@@ -4,7 +4,7 @@
 ``[[M, -sqrt(tau) K], [sqrt(tau) K, M]]`` and the SPD target
 ``H = M + sqrt(tau) K``; ``preconditioner(**fsai_options)`` returns
 ``RepeatedFSAI(FSAI(H))``, which applies the scalar FSAI to both components
-of vec2 arrays through 2 x 2 block products of ``diag(G, G)``.  The lifted
+of vec2 arrays through products of ``diag(G, G)`` that read each entry once.  The lifted
 system is nonsymmetric: solve it with ``linear.gmres`` (never CG/CR).
 """
 
@@ -37,12 +37,12 @@ class RepeatedFSAI(LinearOperator):
         blocks[:, 1, 1] = g.values
         self.G = BsrMatrix(g.nrow, g.ncol, (2, 2), g.offsets, g.columns, blocks)
         self.GT = bsr_transposed(self.G)
+        t_values = self.GT.values[:, 0, 0].contiguous()
         vdt = factor.dtype
         self._op = _lib.new_op(
-            "gbpc_op_fsai", g.nrow, 2, _lib.ptr(self.G.offsets), _lib.ptr(self.G.columns),
-            _lib.ptr(self.G.values), _lib.ptr(self.GT.offsets), _lib.ptr(self.GT.columns),
-            _lib.ptr(self.GT.values), _lib.dtype_code(dt), _lib.dtype_code(vdt),
-            _lib.stream(g.device))
+            "gbpc_op_fsai_pair", g.nrow, _lib.ptr(g.offsets), _lib.ptr(g.columns),
+            _lib.ptr(g.values), _lib.ptr(self.GT.offsets), _lib.ptr(self.GT.columns),
+            _lib.ptr(t_values), _lib.dtype_code(dt), _lib.dtype_code(vdt), _lib.stream(g.device))
         super().__init__((2 * g.nrow, 2 * g.ncol), vdt, g.device, self._apply)
 
     def _apply(self, x, y, z, alpha, beta):

@@ -103,6 +103,7 @@ struct Sell {
   int B = 1;        // block size
   int nslices = 0;
   int vdtype = GBPC_F64;
+  int copies = 1;    // 2: scalar rows, applied to two interleaved vectors
   int64_t nent = 0;  // entries including padding
   int widest = 0;    // at least the width of every slice
   DevBuf slice_ptr;  // int64[nslices + 1]

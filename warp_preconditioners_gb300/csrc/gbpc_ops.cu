@@ -250,7 +250,7 @@ struct FsaiOp : Operator {
   }
   bool apply_widened(const float* x, double* z, const int* guard, const DotSpec* dot,
                      cudaStream_t st, int* rc) override {
-    if (g.B != 1 || vdtype != GBPC_F32) return false;
+    if (g.B != 1 || g.copies != 1 || vdtype != GBPC_F32) return false;
     *rc = sell_spmv(g, vdtype, x, nullptr, tmp.p, 1.0, 0.0, guard, EpiHost{}, nullptr, st);
     if (*rc) return true;
     PdlChain chain;
@@ -262,7 +262,7 @@ struct FsaiOp : Operator {
   }
   bool gathers_x() const override { return false; }
   int scalar_products(const Sell** out, int max) const override {
-    if (max < 2 || g.B != 1 || g.vdtype != GBPC_F64 || gt.vdtype != GBPC_F64 ||
+    if (max < 2 || g.B != 1 || g.copies != 1 || g.vdtype != GBPC_F64 || gt.vdtype != GBPC_F64 ||
         vdtype != GBPC_F64)
       return 0;
     out[0] = &g;
@@ -521,15 +521,11 @@ extern "C" int gbpc_op_sparse(int nrow, int ncol, int block, const int32_t* offs
   return GBPC_OK;
 }
 
-extern "C" int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int32_t* g_col,
-                            const void* g_val, const int32_t* gt_off, const int32_t* gt_col,
-                            const void* gt_val, int value_dtype, int vector_dtype, void* stream,
-                            gbpc_op** out) {
-  NvtxRange nvtx_range("gbpc_op_fsai");
-  if (!out || nrow < 0 || !g_off || !gt_off || block < 1 || block > 4) {
-    gbpc_set_error("gbpc_op_fsai: bad arguments");
-    return GBPC_ERR_ARG;
-  }
+namespace {
+// `copies` > 1: scalar rows (block 1) applied to that many interleaved vectors.
+int make_fsai(int nrow, int block, int copies, const int32_t* g_off, const int32_t* g_col,
+              const void* g_val, const int32_t* gt_off, const int32_t* gt_col, const void* gt_val,
+              int value_dtype, int vector_dtype, void* stream, gbpc_op** out) {
   const bool low = vector_dtype == GBPC_F32_APPLY;
   if (low && value_dtype != GBPC_F32 && value_dtype != GBPC_BF16) {
     gbpc_set_error("float32 application needs float32 or bfloat16 factor storage");
@@ -541,8 +537,8 @@ extern "C" int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int
   if (low) {
     // The float32 operator, wrapped behind float64 vectors.
     gbpc_op* inner = nullptr;
-    rc = gbpc_op_fsai(nrow, block, g_off, g_col, g_val, gt_off, gt_col, gt_val, value_dtype,
-                      GBPC_F32, stream, &inner);
+    rc = make_fsai(nrow, block, copies, g_off, g_col, g_val, gt_off, gt_col, gt_val, value_dtype,
+                   GBPC_F32, stream, &inner);
     if (rc) return rc;
     auto* w = new LowPrecisionOp;
     w->inner = std::move(inner->impl);
@@ -550,7 +546,7 @@ extern "C" int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int
     w->device_bytes = w->inner->device_bytes;
     {
       ByteTally tally(&w->device_bytes);
-      w->rows = (int64_t)nrow * block;
+      w->rows = (int64_t)nrow * block * copies;
       w->vdtype = GBPC_F64;
       rc = w->in32.alloc(sizeof(float) * std::max<int64_t>(w->rows, 1));
       if (!rc) rc = w->out32.alloc(sizeof(float) * std::max<int64_t>(w->rows, 1));
@@ -564,11 +560,12 @@ extern "C" int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int
   }
   auto* op = new FsaiOp;
   ByteTally tally(&op->device_bytes);
-  op->rows = (int64_t)nrow * block;
+  op->rows = (int64_t)nrow * block * copies;
   op->vdtype = vector_dtype;
   const int in = input_dtype(value_dtype);
   rc = sell_build(op->g, nrow, nrow, block, g_off, g_col, g_val, in, value_dtype, SellBuild{}, st);
   if (!rc) rc = sell_build(op->gt, nrow, nrow, block, gt_off, gt_col, gt_val, in, value_dtype, SellBuild{}, st);
+  op->g.copies = op->gt.copies = copies;
   if (!rc) rc = op->tmp.alloc(dtype_size(vector_dtype) * std::max<int64_t>(op->rows, 1));
   if (!rc) {
     cudaError_t e = cudaStreamSynchronize(st);
@@ -583,6 +580,33 @@ extern "C" int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int
   }
   GBPC_OUT_OP(op);
   return GBPC_OK;
+}
+}  // namespace
+
+extern "C" int gbpc_op_fsai(int nrow, int block, const int32_t* g_off, const int32_t* g_col,
+                            const void* g_val, const int32_t* gt_off, const int32_t* gt_col,
+                            const void* gt_val, int value_dtype, int vector_dtype, void* stream,
+                            gbpc_op** out) {
+  NvtxRange nvtx_range("gbpc_op_fsai");
+  if (!out || nrow < 0 || !g_off || !gt_off || block < 1 || block > 4) {
+    gbpc_set_error("gbpc_op_fsai: bad arguments");
+    return GBPC_ERR_ARG;
+  }
+  return make_fsai(nrow, block, 1, g_off, g_col, g_val, gt_off, gt_col, gt_val, value_dtype,
+                   vector_dtype, stream, out);
+}
+
+extern "C" int gbpc_op_fsai_pair(int nrow, const int32_t* g_off, const int32_t* g_col,
+                                 const void* g_val, const int32_t* gt_off, const int32_t* gt_col,
+                                 const void* gt_val, int value_dtype, int vector_dtype,
+                                 void* stream, gbpc_op** out) {
+  NvtxRange nvtx_range("gbpc_op_fsai_pair");
+  if (!out || nrow < 0 || !g_off || !gt_off) {
+    gbpc_set_error("gbpc_op_fsai_pair: bad arguments");
+    return GBPC_ERR_ARG;
+  }
+  return make_fsai(nrow, 1, 2, g_off, g_col, g_val, gt_off, gt_col, gt_val, value_dtype,
+                   vector_dtype, stream, out);
 }
 
 extern "C" int gbpc_op_fsai_refill(gbpc_op* h, const int32_t* g_off, const int32_t* g_col,

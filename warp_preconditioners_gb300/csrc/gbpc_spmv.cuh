@@ -481,6 +481,117 @@ sell_spmv_bpipe_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A b
   if (DOT) reduce_and_finalize(red, dot_part);
 }
 
+// Scalar rows applied to two interleaved vectors (the product with m (x) I_2),
+// software-pipelined like the scalar kernel.  The one-slice kernel on 2 x 2
+// blocks reads 36 bytes and issues four multiply-adds an entry, two of them
+// with a stored zero; here it is 12 bytes and two, and both components of x
+// come with one load where x is aligned for it.  Sums, rows and slices are the
+// blocked kernel's, so the bits are: a product with a stored zero changes a
+// finite sum in nothing, and a component that is infinite or NaN still turns
+// the other one's sum into NaN (tested on the integer pipes).  Bound by the
+// launch and the latency of a warp's few slices, then by FP64 issue.
+// FSAI applies (GB300, as 2 x 2 blocks before): 40^3 tet cube, width 8 / 16, 29.5 / 41
+// -> 21 / 25 us; 70^3, width 8, 61 -> 33 us; 62 GMRES steps at 40^3 7.31 ->
+// 6.49 ms, at 70^3 17.6 -> 16.1 ms.
+template <typename A>
+__device__ __forceinline__ uint32_t high_bits(A v) {
+  if constexpr (std::is_same<A, double>::value) return (uint32_t)__double2hiint(v) & 0x7fffffffu;
+  else return __float_as_uint(v) & 0x7fffffffu;
+}
+
+template <typename V, typename A, bool DOT, int CH, bool UNIT = false>
+__global__ void __launch_bounds__(kThreads, 1)
+sell_spmv_pair_kernel(SellView<V> m, const A* x, const A* y, A* z, A alpha, A beta, int flags,
+                      const int* guard, EpiDev<A> ep, Reduction red) {
+  using Pair = typename std::conditional<std::is_same<A, double>::value, double2, float2>::type;
+  constexpr uint32_t kNotFinite = std::is_same<A, double>::value ? 0x7ff00000u : 0x7f800000u;
+  const bool run = UNIT || !(flags & F_ALPHA_ZERO);
+  const bool alpha_one = UNIT || (flags & F_ALPHA_ONE) != 0;
+  const bool beta_zero = UNIT || (flags & F_BETA_ZERO) != 0;
+  const bool aligned = reinterpret_cast<uintptr_t>(x) % sizeof(Pair) == 0;
+  const int lane = threadIdx.x & 31;
+  const int warps_total = gridDim.x * (kThreads / 32);
+  const int t = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  // First schedule entries and chunk before the wait (the matrix is not
+  // written while a solve runs; see the scalar kernel).
+  const int64_t idx = sched_index(0, t, warps_total);
+  const bool any = idx < m.nslices;
+  SliceTask cur{-1, 0, 0}, nxt{-1, 0, 0};
+  int pc[CH];
+  V pv[CH];
+  bool have = false;
+  if (any) {
+    cur = load_task(m.sched, idx);
+    const int64_t nidx = sched_index(1, t, warps_total);
+    if (nidx < m.nslices) nxt = load_task(m.sched, nidx);
+    if (run) {
+      load_chunk<V, CH>(m, cur, 0, lane, pc, pv);
+      have = true;
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (guard_off(guard)) return;
+  double dot_part = 0.0;
+  if (any) {
+    int i = 0;
+    while (true) {
+      A acc[2] = {A(0), A(0)};
+      uint32_t top[2] = {0u, 0u};
+      if (run) {
+        if (!have) load_chunk<V, CH>(m, cur, 0, lane, pc, pv);
+        have = false;
+        for (int k0 = 0; k0 < cur.width; k0 += CH) {  // uniform across the warp
+          int c[CH];
+          V v[CH];
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            c[j] = pc[j];
+            v[j] = pv[j];
+          }
+          if (k0 + CH < cur.width) {
+            load_chunk<V, CH>(m, cur, k0 + CH, lane, pc, pv);
+          } else if (nxt.s >= 0) {
+            load_chunk<V, CH>(m, nxt, 0, lane, pc, pv);
+            have = true;
+          }
+          Pair xv[CH];
+          if (aligned) {
+#pragma unroll
+            for (int j = 0; j < CH; ++j)
+              xv[j] = (c[j] >= 0) ? __ldg(reinterpret_cast<const Pair*>(x) + c[j]) : Pair{A(0), A(0)};
+          } else {
+#pragma unroll
+            for (int j = 0; j < CH; ++j)
+              xv[j] = (c[j] >= 0) ? Pair{__ldg(x + 2 * (int64_t)c[j]), __ldg(x + 2 * (int64_t)c[j] + 1)}
+                                  : Pair{A(0), A(0)};
+          }
+#pragma unroll
+          for (int j = 0; j < CH; ++j) {
+            top[0] = max(top[0], high_bits(xv[j].x));
+            top[1] = max(top[1], high_bits(xv[j].y));
+            if (k0 + j < cur.width) {
+              const A a = widen_value<A, V>(v[j]);
+              acc[0] = fma_t<A>(a, xv[j].x, acc[0]);
+              acc[1] = fma_t<A>(a, xv[j].y, acc[1]);
+            }
+          }
+        }
+        if (top[1] >= kNotFinite) acc[0] = A(NAN);
+        if (top[0] >= kNotFinite) acc[1] = A(NAN);
+      }
+      spmv_finish<2, V, A, EPI_AXPBY, DOT>(m, cur.s * kSlice + lane, acc, y, z, alpha, beta, run,
+                                           alpha_one, beta_zero, ep, red, dot_part);
+      if (nxt.s < 0) break;
+      cur = nxt;
+      ++i;
+      const int64_t nidx = sched_index(i + 1, t, warps_total);
+      nxt = nidx < m.nslices ? load_task(m.sched, nidx) : SliceTask{-1, 0, 0};
+    }
+  }
+  if (DOT) reduce_and_finalize(red, dot_part);
+}
+
 // ---------------------------------------------------------------------------
 // Scalar rows with the matrix streamed by the bulk-copy engine.
 //
@@ -893,6 +1004,19 @@ static void launch_spmv(const Sell& m, const void* x, const void* y, void* z, do
                                         red, m.nslices, st);
 }
 
+template <typename V, typename A, bool DOT>
+static void launch_pair(const Sell& m, const void* x, const void* y, void* z, double alpha,
+                        double beta, const int* guard, const Reduction& red, cudaStream_t st) {
+  SellView<V> view{m.nrow, m.nslices, m.slice_ptr.as<int64_t>(), m.cols.as<int32_t>(),
+                   m.vals.as<V>(), m.perm.p ? m.perm.as<int32_t>() : nullptr,
+                   m.sched.as<int4>(), 0, m.err.as<int>()};
+  const int flags = spmv_flags(alpha, beta);
+  auto kern = flags == kUnitFlags ? sell_spmv_pair_kernel<V, A, DOT, 4, true>
+                                  : sell_spmv_pair_kernel<V, A, DOT, 4, false>;
+  launch_k(kern, spmv_grid(m.nslices, 1), kThreads, 0, st, view, (const A*)x, (const A*)y, (A*)z,
+           (A)alpha, (A)beta, flags, guard, EpiDev<A>{}, red);
+}
+
 // Epilogue dispatch.  Triangular-sweep epilogues exist only for V == A,
 // the factored-operator epilogue only for scalar rows.
 template <int B, typename V, typename A>
@@ -945,6 +1069,15 @@ static int spmv_dispatch(const Sell& m, const void* x, const void* y, void* z, d
                          cudaStream_t st) {
   auto by_block = [&](auto vtag) -> int {
     using V = decltype(vtag);
+    if (m.copies == 2) {
+      if (ep.kind != EPI_AXPBY) {
+        gbpc_set_error("unsupported product epilogue %d for two vectors", ep.kind);
+        return GBPC_ERR_ARG;
+      }
+      if (red.w != nullptr) launch_pair<V, A, true>(m, x, y, z, alpha, beta, guard, red, st);
+      else launch_pair<V, A, false>(m, x, y, z, alpha, beta, guard, red, st);
+      return GBPC_OK;
+    }
     switch (m.B) {
       case 1: return dispatch_epi<1, V, A>(m, x, y, z, alpha, beta, guard, ep, red, st);
       case 2: return dispatch_epi<2, V, A>(m, x, y, z, alpha, beta, guard, ep, red, st);
