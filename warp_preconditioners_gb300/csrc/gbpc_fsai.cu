@@ -795,6 +795,170 @@ fsai_round_score_kernel(RoundState<T> R, int cur, const int32_t* __restrict__ of
   }
 }
 
+// w = L^-1 a (row by row), with pivot -= w.w and rhs -= w.v on the way, and
+// w = L^-T v: the two solves of a round for one row, the factor's entries
+// strided by nc (rows of a warp next to each other), w by nt in shared memory.
+//
+// AHEAD loads a batch of 8 entries of L (and each row's diagonal, a and v)
+// before the sequential subtractions of the batch before it; otherwise a
+// batch's loads come right before its own subtractions.  AHEAD is for rounds
+// that leave the GPU short of warps (small matrices, and the last rounds,
+// when few rows still grow): a warp there waits a round trip to L2 or HBM for
+// every 16 FP64 instructions.  Constructor, width 48 (GB300): 24^3 tet cube,
+// step 2, 9.8 -> 7.95 ms; 33^3, step 2, 16.1 -> 14.7; 45^3, step 1, 27.0 ->
+// 25.5.  With every third warp or more at work the other warps cover the
+// wait and the loads ahead cost (45^3, step 2, AHEAD always 29.9 ms, up to
+// all threads 30.2, up to half of them 29.8, up to a third 29.2, never 29.2).
+template <bool AHEAD, typename T>
+__device__ __forceinline__ void forward_solve(const T* Lj, const T* ak, const T* vj, int64_t nc,
+                                              int size, T* w, int nt, T& pivot, T& rhs) {
+  if constexpr (AHEAD) {
+    // Rows of L in batches of 8 entries, each batch (and each row's
+    // diagonal, a and v) loaded before the (sequential) subtractions
+    // of the one before it.
+    const T* Lrow = Lj;  // L(p, q) at Lrow[q nc]
+    T l[8], dp = Lj[0], ap = ak[0], vp = vj[0];
+    for (int p = 0; p < size; ++p) {
+      T acc = ap;
+      const T d = dp, v = vp;
+      const T* Lnext = Lrow + (size_t)(p + 1) * nc;
+      if (p + 1 < size) {
+        dp = Lnext[(size_t)(p + 1) * nc];
+        ap = ak[(size_t)(p + 1) * nc];
+        vp = vj[(size_t)(p + 1) * nc];
+      }
+      for (int q = 0;; q += 8) {
+        const bool last = q + 8 >= p;
+        T ln[8];
+        if (!last) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u)
+            ln[u] = q + 8 + u < p ? Lrow[(size_t)(q + 8 + u) * nc] : T(0);
+        } else if (p + 1 < size) {
+#pragma unroll
+          for (int u = 0; u < 8; ++u) ln[u] = u <= p ? Lnext[(size_t)u * nc] : T(0);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          if (q + u >= p) break;
+          const T t = l[u] * w[(q + u) * nt];
+          acc = acc - t;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) l[u] = ln[u];
+        if (last) break;
+      }
+      Lrow = Lnext;
+      const T wp = acc / d;
+      w[p * nt] = wp;
+      const T sq = wp * wp;
+      pivot = pivot - sq;
+      const T pr = wp * v;
+      rhs = rhs - pr;
+    }
+  } else {
+    for (int p = 0; p < size; ++p) {
+      T acc = ak[(size_t)p * nc];
+      const T* Lrow = Lj + (size_t)(p * (p + 1) / 2) * nc;  // L(p, q) at Lrow[q nc]
+      const T dp = Lrow[(size_t)p * nc];
+      int q = 0;
+      // Loads in batches of 8 ahead of the (sequential) subtractions.
+      for (; q + 8 <= p; q += 8) {
+        T l[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) l[u] = Lrow[(size_t)(q + u) * nc];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const T t = l[u] * w[(q + u) * nt];
+          acc = acc - t;
+        }
+      }
+      for (; q < p; ++q) {
+        const T t = Lrow[(size_t)q * nc] * w[q * nt];
+        acc = acc - t;
+      }
+      const T wp = acc / dp;
+      w[p * nt] = wp;
+      const T sq = wp * wp;
+      pivot = pivot - sq;
+      const T pr = wp * vj[(size_t)p * nc];
+      rhs = rhs - pr;
+    }
+  }
+}
+
+template <bool AHEAD, typename T>
+__device__ __forceinline__ void back_solve(const T* Lj, const T* vj, int64_t nc, int size, T* w,
+                                           int nt) {
+  auto L = [&](int r, int p) -> const T& { return Lj[((size_t)(r * (r + 1) / 2 + p)) * nc]; };
+  if constexpr (AHEAD) {
+    // Columns in batches of 8, each loaded a batch ahead.
+    if (size > 0) {
+      T l[8], dp = L(size - 1, size - 1), vp = vj[(size_t)(size - 1) * nc];
+      for (int p = size - 1; p >= 0; --p) {
+        T acc = vp;
+        const T d = dp;
+        if (p > 0) {
+          dp = L(p - 1, p - 1);
+          vp = vj[(size_t)(p - 1) * nc];
+        }
+        for (int q = p + 1;; q += 8) {
+          const bool last = q + 8 >= size;
+          T ln[8];
+          // The next batch: L(q + 8 ..., p), or L(p ..., p - 1).
+          const int qn = last ? p : q + 8, col = last ? p - 1 : p;
+          if (col >= 0) {
+            int kk = qn * (qn + 1) / 2 + col;  // packed index of L(qn, col)
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              ln[u] = qn + u < size ? Lj[(size_t)kk * nc] : T(0);
+              kk += qn + u + 1;
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            if (q + u >= size) break;
+            const T t = l[u] * w[(q + u) * nt];
+            acc = acc - t;
+          }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) l[u] = ln[u];
+          if (last) break;
+        }
+        w[p * nt] = acc / d;
+      }
+    }
+  } else {
+    for (int p = size - 1; p >= 0; --p) {
+      T acc = vj[(size_t)p * nc];
+      const T dp = L(p, p);
+      int q = p + 1;
+      int k0 = q * (q + 1) / 2 + p;  // packed index of L(q, p)
+      for (; q + 8 <= size; q += 8) {
+        T l[8];
+        int kk = k0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          l[u] = Lj[(size_t)kk * nc];
+          kk += q + u + 1;
+        }
+        k0 = kk;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const T t = l[u] * w[(q + u) * nt];
+          acc = acc - t;
+        }
+      }
+      for (; q < size; ++q) {
+        const T t = Lj[(size_t)k0 * nc] * w[q * nt];
+        acc = acc - t;
+        k0 += q + 1;
+      }
+      w[p * nt] = acc / dp;
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 fsai_round_factor_kernel(RoundState<T> R, int cur, T tolerance, T pivot_floor) {
@@ -804,6 +968,7 @@ fsai_round_factor_kernel(RoundState<T> R, int cur, T tolerance, T pivot_floor) {
   const int W = R.W, S = R.S;
   const int64_t nc = R.nc;
   const int count = R.count[cur];
+  const bool ahead = count <= (int)(gridDim.x * nt / 3);
   const int32_t* list = cur ? R.list1 : R.list0;
   int32_t* next = cur ? R.list0 : R.list1;
   T* w = ws + tid;
@@ -826,33 +991,8 @@ fsai_round_factor_kernel(RoundState<T> R, int cur, T tolerance, T pivot_floor) {
           const T* ak = R.a + (size_t)k * W * nc + j;
           T pivot = T(1);
           T rhs = T(0);
-          for (int p = 0; p < size; ++p) {
-            T acc = ak[(size_t)p * nc];
-            const T* Lrow = Lj + (size_t)(p * (p + 1) / 2) * nc;  // L(p, q) at Lrow[q nc]
-            const T dp = Lrow[(size_t)p * nc];
-            int q = 0;
-            // Loads in batches of 8 ahead of the (sequential) subtractions.
-            for (; q + 8 <= p; q += 8) {
-              T l[8];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) l[u] = Lrow[(size_t)(q + u) * nc];
-#pragma unroll
-              for (int u = 0; u < 8; ++u) {
-                const T t = l[u] * w[(q + u) * nt];
-                acc = acc - t;
-              }
-            }
-            for (; q < p; ++q) {
-              const T t = Lrow[(size_t)q * nc] * w[q * nt];
-              acc = acc - t;
-            }
-            const T wp = acc / dp;
-            w[p * nt] = wp;
-            const T sq = wp * wp;
-            pivot = pivot - sq;
-            const T pr = wp * vj[(size_t)p * nc];
-            rhs = rhs - pr;
-          }
+          if (ahead) forward_solve<true>(Lj, ak, vj, nc, size, w, nt, pivot, rhs);
+          else forward_solve<false>(Lj, ak, vj, nc, size, w, nt, pivot, rhs);
           if (pivot <= pivot_floor || !isfinite(pivot)) {
             stopped = true;
             break;
@@ -865,33 +1005,8 @@ fsai_round_factor_kernel(RoundState<T> R, int cur, T tolerance, T pivot_floor) {
           ++size;
         }
         // L^T z = v, in the reference's order.
-        for (int p = size - 1; p >= 0; --p) {
-          T acc = vj[(size_t)p * nc];
-          const T dp = L(p, p);
-          int q = p + 1;
-          int k0 = q * (q + 1) / 2 + p;  // packed index of L(q, p)
-          for (; q + 8 <= size; q += 8) {
-            T l[8];
-            int kk = k0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              l[u] = Lj[(size_t)kk * nc];
-              kk += q + u + 1;
-            }
-            k0 = kk;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const T t = l[u] * w[(q + u) * nt];
-              acc = acc - t;
-            }
-          }
-          for (; q < size; ++q) {
-            const T t = Lj[(size_t)k0 * nc] * w[q * nt];
-            acc = acc - t;
-            k0 += q + 1;
-          }
-          w[p * nt] = acc / dp;
-        }
+        if (ahead) back_solve<true>(Lj, vj, nc, size, w, nt);
+        else back_solve<false>(Lj, vj, nc, size, w, nt);
         for (int p = 0; p < size; ++p) R.z[(size_t)j * W + p] = w[p * nt];
         R.size[j] = size;
         if (stopped) {

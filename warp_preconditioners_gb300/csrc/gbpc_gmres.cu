@@ -330,7 +330,7 @@ __device__ __forceinline__ void coefficients(const double* partials, unsigned cl
 // (GB300): 17^3 tet cube 5.39 -> 5.05 ms, 40^3 (128,000 unknowns) 8.11 -> 7.31,
 // 70^3 18.4 -> 17.6 against four passes over the basis whose last CTAs
 // finish each sum; with the update and the dot products kept apart and only
-// the sums moved, 70^3 took 0.7 ms more than before.
+// the sums moved, 40^3 / 70^3 took 0.4 / 1.3 ms more than fused.
 template <bool UPDATE>
 __global__ void __cluster_dims__(kGCluster, 1, 1) __launch_bounds__(kGT, kMdotCtas / kSms)
 gm_mdot_kernel(int64_t n, const double* V, double* w, GmresState* s, GmresWork wk, const double* in,
